@@ -126,6 +126,7 @@ void release(xpbd_ctx* c) {
     c->patch_ver.release(); c->xv.release(); c->vperm.release(); c->pverts_v.release(); c->faces_v.release();
     c->vdeg_p.release(); c->vdeg_c.release(); c->factive.release(); c->vface_off.release(); c->vface.release();
     c->fcol_d.release(); c->cm_off.release(); c->n_ctasks.release(); c->ctask.release(); c->cface.release();
+    c->cl_tab.release(); c->cl_ifl.release(); c->cl_ifo.release(); c->cl_act_faces.release(); c->cl_act_off.release();
     c->res_partial.release(); c->res_rows.release(); c->energy_partial.release(); c->rvec.release();
     c->mlp_p.release(); c->mlp_m.release(); c->mlp_v.release(); c->mlp_g.release(); c->mlp_w4f.release();
     c->mlp_tiles.release(); c->mat.release(); c->feat.release(); c->pred.release(); c->target.release();
@@ -170,14 +171,17 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
     std::vector<int> voff(V + 1, 0);
     for (int q = 0; q < P; q++)
         for (int k = 0; k < (pmeta[q].y >> 8); k++) voff[pv(q, k) + 1]++;
+    // the versioned sweep orders itself by vertex versions: only where a vertex
+    // has more patches than its fields hold (below) does it need the lists
+    const bool lists = c->prm.gs_variant != 4 || *std::max_element(voff.begin(), voff.end()) > 255;
     for (int v = 0; v < V; v++) voff[v + 1] += voff[v];
-    std::vector<int> vt(voff[V]), fill(voff.begin(), voff.end() - 1);
-    for (int q = 0; q < P; q++)
+    std::vector<int> vt(lists ? voff[V] : 0), fill(voff.begin(), voff.end() - 1);
+    for (int q = 0; q < P && lists; q++)
         for (int k = 0; k < (pmeta[q].y >> 8); k++) vt[fill[pv(q, k)]++] = task_of[q];
     // per-task dependency lists
     std::vector<int> doff(NT + 1, 0), dep;
     std::vector<int> scratch;
-    for (int j = 0; j < NT; j++) {
+    for (int j = 0; j < NT && lists; j++) {
         scratch.clear();
         for (int q = tasks[j].x; q < tasks[j].x + tasks[j].y; q++)
             for (int k = 0; k < (pmeta[q].y >> 8); k++) {
@@ -415,6 +419,443 @@ int build_flow_contacts(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::
     XPBD_CU(c, cudaMemcpy(c->vface.p, ent.data(), sizeof(int) * ent.size(), cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->fcol_d.p, fcol.data(), sizeof(int) * F, cudaMemcpyHostToDevice));
     c->flow_contacts = true;
+    return XPBD_OK;
+}
+
+// Tables of the on-chip sweep, where the mesh is small enough for it: every
+// instance becomes one cluster of csize blocks, which share its patches by
+// rest position: slabs across an axis, or recursive bisection. A colour of
+// which some block has more than kClusterLanes patches (one warp per scheduler,
+// so a phase costs the latency of one patch) is split into as many rounds;
+// its patches share no vertex, so that changes nothing. On GB300 a round takes
+// 1.1 us with one block and 1.4 us with several (1.65 and 2.2 us in the separate
+// form), 0.75 us more where it waits for another block; the versioned sweep
+// takes 2.2-2.5 us a colour, the colour launches of the separate form 2.9 us.
+// Size and shape are those of the least such sum whose data fit the shared
+// memory. Leaves cluster_on off when there is none below the other route's.
+// hm: the tet records m0, m1, m2 in slot order.
+int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector<int4>& pverts,
+                  const std::vector<double>& X, const std::vector<float4>* const hm[3],
+                  const std::vector<int>& fcol, const std::vector<int>& finst) {
+    c->cluster_on = c->cluster_contacts = false;
+    const int P = (int)pmeta.size(), V = c->V, F = c->F, K = c->n_inst;
+    int ncol = c->n_tet_colours;
+    const bool separate = c->prm.constraint_type == XPBD_CONSTRAINT_SEPARATE;
+    int dev = 0, sms = 0;
+    XPBD_CU(c, cudaGetDevice(&dev));
+    XPBD_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (ncol > kMaxClusterColours || (F && c->n_face_colours > kMaxFlowFaceColours) || K > sms ||
+        P > 2LL * kMaxClusterSize * kClusterLanes * ncol * K)
+        return XPBD_OK;
+    auto pv = [&](int q, int k) {
+        const int4& a = pverts[2 * (size_t)q + (k >> 2)];
+        const int kk = k & 3;
+        return kk == 0 ? a.x : (kk == 1 ? a.y : (kk == 2 ? a.z : a.w));
+    };
+    // each instance's patches, their rest centroids
+    std::vector<std::vector<int>> mine(K);
+    std::vector<double> centre(3 * (size_t)P, 0.0);
+    for (int q = 0; q < P; q++) {
+        const int64_t t = c->tet_of_slot[pmeta[q].x];
+        mine[std::upper_bound(c->toff.begin(), c->toff.end(), t) - c->toff.begin() - 1].push_back(q);
+        const int n = pmeta[q].y >> 8;
+        for (int k = 0; k < n; k++)
+            for (int i = 0; i < 3; i++) centre[3 * (size_t)q + i] += X[3 * (size_t)pv(q, k) + i] / n;
+    }
+    // per patch and vertex slot the patches around the vertex and those of a
+    // lower colour (slot order is colour order, and a colour holds a vertex once)
+    std::vector<int> deg(V, 0);
+    std::vector<int4> ver(P, make_int4(0, 0, 0, 0));
+    for (int pass = 0; pass < 2; pass++) {
+        std::vector<int> seen_v(V, 0);
+        for (int q = 0; q < P; q++)
+            for (int k = 0; k < (pmeta[q].y >> 8); k++) {
+                const int v = pv(q, k);
+                if (pass == 0) {
+                    if (++deg[v] > 255) return XPBD_OK;
+                } else {
+                    (&ver[q].x)[k >> 1] |= (deg[v] << 8 | seen_v[v]++) << (16 * (k & 1));
+                }
+            }
+    }
+    // vertices in the order in which runs of 32 patches first touch them, corner
+    // by corner, lane by lane
+    std::vector<int> rank(V, -1);
+    int ranks = 0;
+    for (int q0 = 0; q0 < P; q0 += 32)
+        for (int k = 0; k < kMaxPatchVerts; k++)
+            for (int q = q0; q < std::min(P, q0 + 32); q++)
+                if (k < (pmeta[q].y >> 8) && rank[pv(q, k)] < 0) rank[pv(q, k)] = ranks++;
+    // pieces of [first, last) of an instance's patches into blocks b .. b + n - 1
+    std::vector<int> block(P, 0);
+    auto bisect = [&](auto&& self, std::vector<int>& list, size_t first, size_t last, int b, int n) -> void {
+        if (n == 1) {
+            for (size_t i = first; i < last; i++) block[list[i]] = b;
+            return;
+        }
+        double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+        for (size_t i = first; i < last; i++)
+            for (int k = 0; k < 3; k++) {
+                lo[k] = std::min(lo[k], centre[3 * (size_t)list[i] + k]);
+                hi[k] = std::max(hi[k], centre[3 * (size_t)list[i] + k]);
+            }
+        int ax = 0;
+        for (int k = 1; k < 3; k++)
+            if (hi[k] - lo[k] > hi[ax] - lo[ax]) ax = k;
+        const size_t mid = first + (last - first) / 2;
+        std::nth_element(list.begin() + first, list.begin() + mid, list.begin() + last, [&](int a, int d) {
+            const double u = centre[3 * (size_t)a + ax], v = centre[3 * (size_t)d + ax];
+            return u < v || (u == v && a < d);
+        });
+        self(self, list, first, mid, b, n / 2);
+        self(self, list, mid, last, b + n / 2, n / 2);
+    };
+    std::vector<int> pcol(P);
+    for (int col = 0; col < ncol; col++)
+        for (int q = c->pcol_off[col]; q < c->pcol_off[col + 1]; q++) pcol[q] = col;
+    // n slabs across axis ax, the cuts moved to the nearest step of the
+    // coordinate (a layer of a grid) within half a slab
+    std::vector<std::vector<int>> by_axis[3];
+    auto slabs = [&](int ax, int n) {
+        auto at = [&](int q) { return centre[3 * (size_t)q + ax]; };
+        if (by_axis[ax].empty()) {
+            by_axis[ax] = mine;
+            for (auto& l : by_axis[ax])
+                std::sort(l.begin(), l.end(), [&](int a, int d) { return at(a) < at(d) || (at(a) == at(d) && a < d); });
+        }
+        for (int k = 0; k < K; k++) {
+            const std::vector<int>& l = by_axis[ax][k];
+            const long long m = (long long)l.size();
+            const double eps = 1e-6 * (at(l.back()) - at(l.front()));
+            long long lo = 0;
+            for (int r = 0; r < n; r++) {
+                long long hi = m * (r + 1) / n;
+                for (long long d = 0; r + 1 < n && 2 * n * d <= m; d++) {
+                    const long long up = hi + d, down = hi - d;
+                    if (up < m && at(l[up]) - at(l[up - 1]) > eps) { hi = up; break; }
+                    if (down > lo && at(l[down]) - at(l[down - 1]) > eps) { hi = down; break; }
+                }
+                for (long long i = lo; i < hi; i++) block[l[i]] = k * n + r;
+                lo = std::max(lo, hi);
+            }
+        }
+    };
+    // shape 0-2: slabs across that axis; 3: recursive bisection (n a power of two)
+    std::vector<int> cnt;
+    auto assign = [&](int shape, int n) {  // -> the most patches of one colour in a block
+        if (shape < 3) slabs(shape, n);
+        else for (int k = 0; k < K; k++) bisect(bisect, mine[k], 0, mine[k].size(), k * n, n);
+        cnt.assign((size_t)K * n * ncol, 0);
+        int worst = 0;
+        for (int q = 0; q < P; q++) worst = std::max(worst, ++cnt[(size_t)block[q] * ncol + pcol[q]]);
+        return worst;
+    };
+    // colours with a vertex that another block wrote in the colour before: their
+    // phases wait for it (about 0.75 us on GB300; a write two phases back is there)
+    auto stalls = [&]() {
+        std::vector<int> first(V, -1), last(V, -1);
+        std::vector<char> s(ncol, 0);
+        for (int q = 0; q < P; q++)
+            for (int k = 0; k < (pmeta[q].y >> 8); k++) {
+                const int v = pv(q, k), l = last[v];
+                if (l < 0) first[v] = q;
+                else if (block[l] != block[q] && pcol[l] + 1 == pcol[q]) s[pcol[q]] = 1;
+                last[v] = q;
+            }
+        for (int v = 0; v < V; v++)
+            if (last[v] >= 0 && pcol[first[v]] == 0 && pcol[last[v]] == ncol - 1 && block[first[v]] != block[last[v]])
+                s[0] = 1;
+        return (int)std::count(s.begin(), s.end(), 1);
+    };
+    size_t largest = 0;
+    for (int k = 0; k < K; k++) largest = std::max(largest, mine[k].size());
+    struct Choice {
+        double us;
+        int n, shape;
+    };
+    std::vector<Choice> choices;
+    const double other = separate ? 2.9 : 2.2;
+    const int n_min = (int)std::min<size_t>(kMaxClusterSize, (largest + kClusterLanes * ncol - 1) / (kClusterLanes * ncol));
+    for (int n : {n_min, n_min + 1, n_min + 2, n_min + 4, kMaxClusterSize}) {
+        if (n > kMaxClusterSize || (K > 1 && K * n > sms) || (!choices.empty() && choices.back().n == n)) continue;
+        for (int sh = 0; sh < 4; sh++) {
+            if ((n == 1 && sh > 0) || (sh == 3 && (n & (n - 1)))) continue;
+            assign(sh, n);
+            double us = 0;
+            for (int col = 0; col < ncol; col++) {
+                int most = 1;
+                for (int b = 0; b < K * n; b++) most = std::max(most, cnt[(size_t)b * ncol + col]);
+                us += (n == 1 ? (separate ? 1.65 : 1.1) : (separate ? 2.2 : 1.4)) *
+                      ((most + kClusterLanes - 1) / kClusterLanes);
+            }
+            if (us < other * ncol && n > 1) us += 0.75 * stalls();
+            choices.push_back(Choice{us, n, sh});
+        }
+    }
+    std::stable_sort(choices.begin(), choices.end(), [](const Choice& a, const Choice& b) { return a.us < b.us; });
+    const int colours = ncol;
+    const std::vector<int> colour_of = pcol;
+    for (const Choice& ch : choices) {
+        if (ch.us >= other * colours) break;
+        ncol = colours;
+        pcol = colour_of;
+        assign(ch.shape, ch.n);
+        const int csize = ch.n, ncta = K * csize;
+        {
+            // rounds: the i-th of a block's n patches of a colour in round i * rounds / n
+            std::vector<int> first(colours), rounds(colours, 1), at((size_t)ncta * colours, 0);
+            int total = 0;
+            for (int col = 0; col < colours; col++) {
+                for (int b = 0; b < ncta; b++)
+                    rounds[col] = std::max(rounds[col], (cnt[(size_t)b * colours + col] + kClusterLanes - 1) / kClusterLanes);
+                first[col] = total;
+                total += rounds[col];
+            }
+            if (total > kMaxClusterColours) continue;
+            for (int q = 0; q < P; q++) {
+                const int col = colour_of[q];
+                const size_t e = (size_t)block[q] * colours + col;
+                pcol[q] = first[col] + (int)((long long)at[e]++ * rounds[col] / cnt[e]);
+            }
+            ncol = total;
+            cnt.assign((size_t)ncta * ncol, 0);
+            for (int q = 0; q < P; q++) cnt[(size_t)block[q] * ncol + pcol[q]]++;
+        }
+        // patches by block and colour, in slot order
+        std::vector<int> off((size_t)ncta * ncol + 1, 0);
+        for (size_t i = 0; i < cnt.size(); i++) off[i + 1] = off[i] + cnt[i];
+        std::vector<int> list(P), fill(off.begin(), off.end() - 1);
+        for (int q = 0; q < P; q++) list[fill[(size_t)block[q] * ncol + pcol[q]]++] = q;
+        ClusterShape s{};
+        s.ncta = ncta; s.csize = csize; s.ncol = ncol; s.nfcol = c->n_face_colours;
+        s.threads = kClusterThreads;
+        std::vector<int4> part(2 * (size_t)ncta), range((size_t)ncta * ncol), vidx(P), meta(P);
+        std::vector<int> slots(P);
+        std::vector<int4> vers(P);
+        std::vector<float4> recs(3 * (size_t)c->T);
+        int nrec = 0;
+        // the blocks' vertices: which of them hold each vertex (at most nine)
+        constexpr int kCopies = 9;
+        std::vector<int> copy((size_t)V * kCopies, -1), copies(V, 0), local((size_t)V * kCopies, 0);
+        bool ok = true;
+        for (int q = 0; q < P && ok; q++)
+            for (int k = 0; k < (pmeta[q].y >> 8); k++) {
+                const int v = pv(q, k);
+                int* m = &copy[(size_t)v * kCopies];
+                int j = 0;
+                while (j < copies[v] && m[j] != block[q]) j++;
+                if (j < copies[v]) continue;
+                if (j == kCopies) { ok = false; break; }
+                m[copies[v]++] = block[q];
+            }
+        if (!ok) continue;
+        auto slot_in = [&](int v, int b) {
+            int j = 0;
+            while (copy[(size_t)v * kCopies + j] != b) j++;
+            return (size_t)v * kCopies + j;
+        };
+        std::vector<int> verts;
+        std::vector<uint4> remote;
+        std::vector<char> seen(V, 0);  // per block: 1 numbered
+        bool generic = false;
+        size_t max_rec = 0;
+        for (int b = 0; b < ncta; b++) {
+            const int p0 = off[(size_t)b * ncol], p1 = off[(size_t)(b + 1) * ncol];
+            const int v0 = (int)verts.size(), r0 = (int)remote.size();
+            int nv = 0, nb = 0, nt = 0;
+            // shared vertices first, in one order for all blocks, so that the
+            // lanes of a warp write neighbouring rows of a neighbour's copies;
+            // then the rest, in the order in which the lanes of a colour first
+            // touch them, corner by corner: a warp reads neighbouring rows
+            auto number = [&](int v) {
+                local[slot_in(v, b)] = nv++;
+                int owner = copy[(size_t)v * kCopies];
+                for (int j = 1; j < copies[v]; j++) owner = std::min(owner, copy[(size_t)v * kCopies + j]);
+                verts.push_back(owner == b ? (int)(0x80000000u | (unsigned)v) : v);
+            };
+            std::vector<int> common;
+            for (int i = p0; i < p1; i++)
+                for (int k = 0; k < (pmeta[list[i]].y >> 8); k++) {
+                    const int v = pv(list[i], k);
+                    if (!seen[v] && copies[v] > 1) common.push_back(v);
+                    if (copies[v] > 1) seen[v] = 1;
+                }
+            std::sort(common.begin(), common.end(), [&](int u, int v) { return rank[u] < rank[v]; });
+            for (int v : common) number(v);
+            nb = nv;
+            for (int col = 0; col < ncol; col++)
+                for (int k = 0; k < kMaxPatchVerts; k++)
+                    for (int i = off[(size_t)b * ncol + col]; i < off[(size_t)b * ncol + col + 1]; i++) {
+                        if (k >= (pmeta[list[i]].y >> 8)) continue;
+                        const int v = pv(list[i], k);
+                        if (!seen[v]) {
+                            seen[v] = 1;
+                            number(v);
+                        }
+                    }
+            for (int i = v0; i < (int)verts.size(); i++) seen[verts[i] & 0x7fffffff] = 0;
+            remote.resize(r0 + nb);
+            if (nv > 65535 || nb >= 4095) ok = false;  // 16-bit local indices, 12-bit ones of the shared vertices
+            for (int col = 0; col < ncol; col++) {
+                const size_t e = (size_t)b * ncol + col;
+                const int t0 = nt;
+                for (int i = off[e]; i < off[e + 1]; i++) {
+                    const int q = list[i], n = pmeta[q].y & 0xff;
+                    slots[i] = pmeta[q].x;
+                    meta[i] = make_int4(nt, pmeta[q].y, pmeta[q].z, pmeta[q].w);
+                    const unsigned long long loc = (unsigned long long)(unsigned)pmeta[q].z |
+                                                   ((unsigned long long)(unsigned)pmeta[q].w << 32);
+                    generic |= pmeta[q].y != (5 | (8 << 8)) || loc != kHexLocA;
+                    for (int k = 0; k < 3; k++)
+                        std::copy(hm[k]->begin() + pmeta[q].x, hm[k]->begin() + pmeta[q].x + n,
+                                  recs.begin() + (size_t)k * c->T + nrec + nt);
+                    vers[i] = ver[q];
+                    nt += n;
+                }
+                range[e] = make_int4(off[e] - p0, cnt[e], nt - t0, t0);
+                max_rec = std::max(max_rec, (size_t)(nt - t0));
+            }
+            part[2 * b] = make_int4(v0, nv, nb, p0);
+            part[2 * b + 1] = make_int4(p1 - p0, r0, nt, nrec);
+            nrec += nt;
+            s.max_nv = std::max(s.max_nv, nv);
+            s.max_nb = std::max(s.max_nb, nb);
+            s.max_p = std::max(s.max_p, p1 - p0);
+            s.max_t = std::max(s.max_t, nt);
+        }
+        if (!ok) continue;
+        for (int b = 0; b < ncta; b++)
+            for (int i = 0; i < part[2 * b].z; i++) {
+                const int v = verts[part[2 * b].x + i] & 0x7fffffff;
+                unsigned short r[kCopies - 1];
+                std::fill(r, r + kCopies - 1, (unsigned short)0xffff);
+                for (int j = 0, n = 0; j < copies[v]; j++) {
+                    const int o = copy[(size_t)v * kCopies + j];
+                    if (o != b) r[n++] = (unsigned short)((o % csize) << 12 | local[(size_t)v * kCopies + j]);
+                }
+                std::memcpy(&remote[part[2 * b + 1].y + i], r, sizeof(uint4));
+            }
+        // what each colour sends to the other blocks
+        std::vector<uint2> send;
+        std::vector<int> send_off((size_t)ncta * (ncol + 1), 0);
+        for (int b = 0; b < ncta && csize > 1; b++) {
+            const size_t first = send.size();
+            for (int col = 0; col <= ncol; col++) {
+                send_off[(size_t)b * (ncol + 1) + col] = (int)send.size();
+                if (col == ncol) break;
+                const size_t e = (size_t)b * ncol + col;
+                for (int k = 0; k < kMaxPatchVerts; k++)
+                    for (int i = off[e]; i < off[e + 1]; i++) {
+                        if (k >= (pmeta[list[i]].y >> 8)) continue;
+                        const int v = pv(list[i], k);
+                        for (int j = 0; j < copies[v]; j++) {
+                            const int o = copy[(size_t)v * kCopies + j];
+                            if (o != b)
+                                send.push_back(make_uint2(
+                                    (unsigned)local[slot_in(v, b)] << 16 | (unsigned)(o % csize) << 12 |
+                                        (unsigned)local[(size_t)v * kCopies + j],
+                                    (unsigned)((&ver[list[i]].x)[k >> 1] >> (16 * (k & 1))) & 0xffffu));
+                        }
+                    }
+            }
+            s.max_send = std::max(s.max_send, (int)(send.size() - first + 3) / 4 * 4);
+        }
+        for (int q = 0; q < P; q++) {
+            int w[4] = {0, 0, 0, 0};
+            for (int k = 0; k < (pmeta[list[q]].y >> 8); k++)
+                w[k >> 1] |= local[slot_in(pv(list[q], k), block[list[q]])] << (16 * (k & 1));
+            vidx[q] = make_int4(w[0], w[1], w[2], w[3]);
+        }
+        // shared memory: vertices, records (all of them, or two buffers of one
+        // colour), topology, copies, multipliers, the generic patches' scratch
+        s.max_t = (s.max_t + 1) / 2 * 2;
+        s.max_nb = (s.max_nb + 3) / 4 * 4;
+        const size_t rest = 16 * (size_t)s.max_nv + (csize > 1 ? 48 : 32) * (size_t)s.max_p +
+                            (csize > 1 ? 28 : 0) * (size_t)s.max_nb + 8 * (size_t)s.max_send + 8 * (size_t)s.max_t + (generic ? 16 * (size_t)kMaxPatchVerts * kClusterLanes : 0);
+        const size_t all = 48 * (size_t)s.max_t, two = 2 * 48 * max_rec;
+        s.resident = rest + all <= (size_t)kClusterSmemMax;
+        s.rec_cap = (int)(s.resident ? (size_t)s.max_t : max_rec);
+        s.smem = rest + (s.resident ? all : two);
+        if (s.smem > (size_t)kClusterSmemMax) continue;
+        // faces: the block that projects a face's contacts holds its three vertices
+        std::vector<int4> fl(F);
+        std::vector<int> fblock(F), cifl(F), cifo;
+        bool fok = F > 0;
+        for (int f = 0; f < F && fok; f++) {
+            const int* e = &c->faces_h[3 * (size_t)f];
+            int home = -1;
+            for (int j = 0; j < copies[e[0]] && home < 0; j++) {
+                const int b = copy[(size_t)e[0] * kCopies + j];
+                bool in = true;
+                for (int k = 1; k < 3; k++) {
+                    const int* m = &copy[(size_t)e[k] * kCopies];
+                    in = in && std::find(m, m + copies[e[k]], b) != m + copies[e[k]];
+                }
+                if (in) home = b;
+            }
+            fok = home >= 0 && home / csize == finst[f];
+            if (!fok) break;
+            fblock[f] = home;
+            fl[f] = make_int4(local[slot_in(e[0], home)], local[slot_in(e[1], home)], local[slot_in(e[2], home)],
+                              deg[e[0]] | deg[e[1]] << 8 | deg[e[2]] << 16);
+        }
+        if (sweep_cluster_fits(s, separate, false) <= 0 || (fok && sweep_cluster_fits(s, separate, true) <= 0)) continue;
+        if (!fok) fl.clear();
+        // one device buffer for the tables
+        std::vector<int4> tab;
+        auto put = [&](const void* p, size_t bytes) {
+            const size_t at = tab.size();
+            tab.resize(at + (bytes + 15) / 16);
+            if (bytes) std::memcpy(&tab[at], p, bytes);
+            return at;
+        };
+        const size_t o_part = put(part.data(), sizeof(int4) * part.size());
+        const size_t o_range = put(range.data(), sizeof(int4) * range.size());
+        const size_t o_vidx = put(vidx.data(), sizeof(int4) * vidx.size());
+        const size_t o_meta = put(meta.data(), sizeof(int4) * meta.size());
+        const size_t o_rem = put(remote.data(), sizeof(uint4) * remote.size());
+        const size_t o_face = put(fl.data(), sizeof(int4) * fl.size());
+        const size_t o_vert = put(verts.data(), sizeof(int) * verts.size());
+        const size_t o_slot = put(slots.data(), sizeof(int) * slots.size());
+        const size_t o_ver = put(vers.data(), sizeof(int4) * vers.size());
+        const size_t o_send = put(send.data(), sizeof(uint2) * send.size());
+        const size_t o_soff = put(send_off.data(), sizeof(int) * send_off.size());
+        const size_t o_rec = put(recs.data(), sizeof(float4) * recs.size());
+        XPBD_CU(c, c->cl_tab.alloc(tab.size() + 1));
+        XPBD_CU(c, cudaMemcpy(c->cl_tab.p, tab.data(), sizeof(int4) * tab.size(), cudaMemcpyHostToDevice));
+        const int4* d = c->cl_tab.p;
+        c->cl = ClusterArrays{d + o_part, d + o_range, d + o_vidx, d + o_meta, d + o_ver, (const int*)(d + o_slot),
+                              (const float4*)(d + o_rec), (size_t)c->T, (const int*)(d + o_vert),
+                              (const uint4*)(d + o_rem), (const uint2*)(d + o_send), (const int*)(d + o_soff),
+                              d + o_face, nullptr, nullptr};
+        c->cl_shape = s;
+        c->cluster_on = true;
+        if (fok) {
+            const int nfc = c->n_face_colours;
+            cifo.assign((size_t)ncta * (nfc + 1), 0);
+            std::vector<int> n((size_t)ncta * nfc, 0);
+            for (int f = 0; f < F; f++) n[(size_t)fblock[f] * nfc + fcol[f]]++;
+            int run = 0;
+            for (int b = 0; b < ncta; b++)
+                for (int col = 0; col <= nfc; col++) {
+                    cifo[(size_t)b * (nfc + 1) + col] = run;
+                    if (col < nfc) run += n[(size_t)b * nfc + col];
+                }
+            std::vector<int> pos(cifo);
+            for (int f = 0; f < F; f++) cifl[pos[(size_t)fblock[f] * (nfc + 1) + fcol[f]]++] = f;
+            XPBD_CU(c, c->cl_ifl.alloc(F));
+            XPBD_CU(c, c->cl_ifo.alloc(cifo.size()));
+            XPBD_CU(c, c->cl_act_faces.alloc(F));
+            XPBD_CU(c, c->cl_act_off.alloc(cifo.size()));
+            XPBD_CU(c, cudaMemcpy(c->cl_ifl.p, cifl.data(), sizeof(int) * F, cudaMemcpyHostToDevice));
+            XPBD_CU(c, cudaMemcpy(c->cl_ifo.p, cifo.data(), sizeof(int) * cifo.size(), cudaMemcpyHostToDevice));
+            XPBD_CU(c, cudaMemset(c->cl_act_off.p, 0, sizeof(int) * cifo.size()));
+            c->cl.act_faces = c->cl_act_faces.p;
+            c->cl.act_off = c->cl_act_off.p;
+            c->cluster_contacts = true;
+        }
+        return XPBD_OK;
+    }
     return XPBD_OK;
 }
 
@@ -860,6 +1301,11 @@ int build(xpbd_ctx* c, const xpbd_mesh_desc* ms, int n_inst) {
             st = build_flow_contacts(c, pmeta, pverts, fcol);
             if (st) return st;
         }
+    }
+    if (!pmeta.empty() && p.solver_type == XPBD_SOLVER_GAUSS_SEIDEL && p.gs_variant == 4) {
+        const std::vector<float4>* const hm[3] = {&hm0, &hm1, &hm2};
+        int st = build_cluster(c, pmeta, pverts, Xcat, hm, fcol, finst);
+        if (st) return st;
     }
     if (!pmeta.empty()) {
         XPBD_CU(c, c->patch_meta.alloc(pmeta.size()));

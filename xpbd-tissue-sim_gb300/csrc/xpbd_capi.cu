@@ -197,6 +197,21 @@ float self_alpha_tilde(const xpbd_ctx* c) {
     return (float)(1e-8 / (c->prm.first_order ? c->prm.dt : c->prm.dt * c->prm.dt));
 }
 
+// Whether the substep's sweeps run on chip (k_sweep_cluster): every static
+// contact and projection of an iteration is in it; latency stamps and the
+// stalled-vertex hook belong to the versioned sweep.
+bool use_cluster(const xpbd_ctx* c) {
+    return c->cluster_on && !c->lat_on && !c->stalled && c->prm.num_iters > 0 &&
+           c->prm.residual_policy != XPBD_RESIDUAL_EVERY_ITERATION && c->att_v.empty() && !c->self_on && !c->nbodies &&
+           (!c->F || c->cluster_contacts);
+}
+
+// A mesh whose largest colour is at most one warp of patches keeps the inertial
+// move, the copies into and out of the sweep's records and the velocities in
+// their own launches: the number of launches a substep of such a mesh makes is
+// part of what the interface reports (xpbd_launch_count).
+bool cluster_fused(const xpbd_ctx* c) { return c->F > 0 || !c->flow_versioned || c->flow_grid > 1; }
+
 // solve_only: XPBDSolver::solve() alone (XPBDSolver.hpp:66-97) -- lambda <- 0
 // and num_iters sweeps on the current positions, with no inertial move, no
 // local collision passes, no fixed reset and no rigid-body update.
@@ -211,12 +226,16 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     cudaStream_t s = c->stream;
     const ContactArrays ca = c->contacts();
     const bool have_faces = c->F > 0;
-    if (!solve_only) {
+    const bool warm = c->warm_mode != XPBD_WARM_NONE;
+    const bool cluster = use_cluster(c);
+    // on chip the inertial move is part of the sweep's launch when nothing
+    // reads the predicted positions before it
+    const bool fuse_predict = cluster && cluster_fused(c) && !solve_only && !track && !warm && !c->record;
+    if (!solve_only && !fuse_predict) {
         Scope sc(c, K_PREDICT);
         if (p.first_order) launch_predict_first_order(c->L(), c->x.p, c->prev.p, c->gdz.p, c->V);
         else launch_predict(c->L(), c->x.p, c->prev.p, c->vel.p, c->V, dt, dz);
     }
-    const bool warm = c->warm_mode != XPBD_WARM_NONE;
     if (track) cudaMemsetAsync(c->res_partial.p, 0, sizeof(double) * (size_t)c->res_stride * (iters + 1), s);
     if (warm) {
         // r(x_pred, 0) before the warm start moves anything
@@ -233,6 +252,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     const bool jacobi = p.solver_type == XPBD_SOLVER_JACOBI;
     const bool local = !solve_only && have_faces && p.num_local_collision_iters > 0 && c->local_slots.p;
     const bool fuse_final = !track && !local && !solve_only;
+    const bool final_on_chip = fuse_predict && fuse_final;
     if (jacobi) {
         const bool gather = p.jacobi_variant == XPBD_JACOBI_GATHER;
         if (track && !every_iter && !warm) exact_residual_row(c, 0, false);
@@ -298,6 +318,25 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
                 Scope sc(c, K_APPLY);
                 launch_apply(c->L(), c->x.p, c->dx.p, c->V, c->prev.p, c->vel.p, last && fuse_final, dt, write_vel);
             }
+        }
+    } else if (cluster) {
+        if (track && !warm) exact_residual_row(c, 0, false);
+        const bool records = !cluster_fused(c);
+        if (records) {
+            Scope sc(c, K_PROJECT_GS);
+            launch_versions_in(c->L(), c->xv.p, c->x.p, c->vperm.p, c->V);
+        }
+        {
+            Scope sc(c, K_PROJECT_GS);
+            const xg::ClusterIo io{c->x.p, c->prev.p, c->vel.p, p.first_order ? c->gdz.p : nullptr,
+                                   records ? c->xv.p : nullptr, c->vperm.p, dt, dz, fuse_predict, final_on_chip,
+                                   write_vel};
+            launch_sweep_cluster(c->L(), c->cl, c->cl_shape, c->tets(), io, iters, !warm, separate, have_faces, ca,
+                                 c->flags.p);
+        }
+        if (records) {
+            Scope sc(c, K_PROJECT_GS);
+            launch_versions_out(c->L(), c->x.p, c->xv.p, c->vperm.p, c->V);
         }
     } else if (!separate && !every_iter && c->att_v.empty() &&
                (!have_faces || (p.gs_variant == 4 && c->flow_versioned && c->flow_contacts && !c->self_on &&
@@ -380,7 +419,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     }
     if (solve_only) return XPBD_OK;
     if (local) enqueue_local_collision_iters(c, p.num_local_collision_iters);
-    if (!jacobi || !fuse_final || iters == 0) {
+    if ((!jacobi || !fuse_final || iters == 0) && !final_on_chip) {
         Scope sc(c, K_FINALIZE);
         launch_finalize(c->L(), c->x.p, c->prev.p, c->vel.p, c->V, dt, write_vel);
     }
@@ -452,17 +491,27 @@ int sync_attachments(xpbd_ctx* c) {
 int prepare_update(xpbd_ctx* c) {
     int ast = sync_attachments(c);
     if (ast) return ast;
-    if (c->F && c->contact_lists_dirty) {
-        // the faces with active static contacts, after the contacts changed
+    // the faces with active static contacts, after the contacts changed, in the
+    // form that the coming substep reads
+    const bool cluster = use_cluster(c);
+    if (c->F && cluster && c->cluster_lists_dirty) {
+        Scope sc(c, K_DETECT);
+        launch_contact_lists(c->L(), c->contacts(), c->cl_ifl.p, c->cl_ifo.p, c->n_face_colours, c->cl_shape.ncta,
+                             c->cl_act_faces.p, c->cl_act_off.p);
+        c->cluster_lists_dirty = false;
+    }
+    if (c->F && (!cluster || c->local_slots.p) && c->contact_lists_dirty) {
         Scope sc(c, K_DETECT);
         launch_contact_lists(c->L(), c->contacts(), c->ifl.p, c->ifo_off.p, c->n_face_colours, c->n_inst,
                              c->act_faces.p, c->act_off.p);
-        if (c->flow_contacts)
-            launch_flow_contact_tables(c->L(), c->contacts(), c->act_faces.p, c->act_off.p, c->n_face_colours,
-                                       c->n_inst, c->vface_off.p, c->vface.p, c->fcol_d.p, c->vdeg_p.p,
-                                       c->factive.p, c->cm_off.p, c->ctask.p, c->n_ctasks.p, c->cface.p,
-                                       c->vdeg_c.p, c->vperm.p, c->V);
         c->contact_lists_dirty = false;
+    }
+    if (c->flow_contacts && !cluster && c->flow_tables_dirty) {
+        Scope sc(c, K_DETECT);
+        launch_flow_contact_tables(c->L(), c->contacts(), c->act_faces.p, c->act_off.p, c->n_face_colours, c->n_inst,
+                                   c->vface_off.p, c->vface.p, c->fcol_d.p, c->vdeg_p.p, c->factive.p, c->cm_off.p,
+                                   c->ctask.p, c->n_ctasks.p, c->cface.p, c->vdeg_c.p, c->vperm.p, c->V);
+        c->flow_tables_dirty = false;
     }
     if (tracking(c) || c->warm_mode != XPBD_WARM_NONE) {
         // one extra row for on-demand residual queries, two for the warm start
@@ -575,7 +624,7 @@ int detect(xpbd_ctx* c) {
         launch_self_detect(c->L(), c->selfs(), c->sgrid, c->x.p, c->faces.p);
     }
     std::fill(c->api_slots.begin(), c->api_slots.end(), -1);  // unknown until read back
-    c->contact_lists_dirty = true;
+    c->contacts_changed();
     return after_launches(c, "detect");
 }
 
@@ -1096,7 +1145,7 @@ int xpbd_clear_collisions(xpbd_ctx* c) {
         XPBD_CU(c, cudaMemsetAsync(c->c_lam.p, 0, sizeof(float) * (size_t)c->S * c->F, c->stream));
         XPBD_CU(c, cudaMemsetAsync(c->rc_count.p, 0, sizeof(int), c->stream));
         if (c->self_on) XPBD_CU(c, cudaMemsetAsync(c->s_n_hits.p, 0, sizeof(int), c->stream));
-        c->contact_lists_dirty = true;
+        c->contacts_changed();
     }
     std::fill(c->api_slots.begin(), c->api_slots.end(), 0);
     return XPBD_OK;
@@ -1136,7 +1185,7 @@ int xpbd_add_static_collision(xpbd_ctx* c, int32_t face, double u, double v, dou
     XPBD_CU(c, cudaMemcpy(c->c_lam.p + slot, &z, sizeof z, cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->c_bary.p + slot, &b, sizeof b, cudaMemcpyHostToDevice));
     c->api_slots[face] = s + 1;
-    c->contact_lists_dirty = true;
+    c->contacts_changed();
     return XPBD_OK;
 }
 
@@ -1426,6 +1475,7 @@ int xpbd_debug_stall_vertex(xpbd_ctx* c, int32_t vertex, int32_t poll_limit) {
     } else {
         c->flow_poll_limit = kFlowLimit;
     }
+    c->stalled = vertex >= 0;
     XPBD_CU(c, cudaMemcpy(c->patch_ver.p, ver.data(), sizeof(int4) * ver.size(), cudaMemcpyHostToDevice));
     c->graph_dirty = true;  // the poll limit is a launch argument
     return XPBD_OK;

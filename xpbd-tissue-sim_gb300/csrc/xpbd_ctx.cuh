@@ -123,6 +123,14 @@ struct xpbd_ctx {
     bool lat_on = false, lat_have = false;
     std::vector<int2> task_inst_h;  // patch task -> first and last instance it touches
     std::vector<int> vperm_h;       // the versioned sweep's vertex numbering (vertex -> record)
+    // Gauss-Seidel on chip (ClusterArrays): one buffer for the static tables,
+    // the per-detection lists beside it
+    bool cluster_on = false, cluster_contacts = false;
+    bool stalled = false;  // xpbd_debug_stall_vertex: the versioned sweep, whose waits it tests, runs
+    xg::ClusterShape cl_shape{};
+    xg::ClusterArrays cl{};
+    DevBuf<int4> cl_tab;
+    DevBuf<int> cl_ifl, cl_ifo, cl_act_faces, cl_act_off;
     DevBuf<float4> c_bary, c_p, c_n;
     DevBuf<float> c_lam;
     int S = 4;
@@ -140,7 +148,10 @@ struct xpbd_ctx {
     // static contacts by instance and face colour: all faces (ifl, ifo_off) and,
     // after each detection, those with an active contact (act_faces, act_off)
     DevBuf<int> ifl, ifo_off, act_faces, act_off;
-    bool contact_lists_dirty = true;
+    // out of date after a detection: the per-instance lists, the versioned
+    // sweep's tables and the on-chip sweep's lists (each built when a route uses it)
+    bool contact_lists_dirty = true, flow_tables_dirty = true, cluster_lists_dirty = true;
+    void contacts_changed() { contact_lists_dirty = flow_tables_dirty = cluster_lists_dirty = true; }
     // self-collisions: grid, binning, hits and contacts (xg::SelfArrays)
     bool self_on = false;
     int n_surf = 0, ncells = 0;

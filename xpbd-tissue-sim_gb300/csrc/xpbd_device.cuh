@@ -561,6 +561,38 @@ __device__ __forceinline__ bool project_one(const TetState<float>& s, const TetA
     return true;
 }
 
+// Static collision projection of one contact slot: C = n.(u x1 + v x2 + w x3 - p),
+// skipped when C > 0, alpha = 0. Returns false when skipped.
+__device__ __forceinline__ bool contact_update(const ContactArrays& c, int slot, const float4 xs[3], float d[3][3],
+                                               float& lam) {
+    const float4 b = c.bary[slot];
+    const float4 p = c.p[slot];
+    const float4 n = c.n[slot];
+    const float a0 = b.x * xs[0].x + b.y * xs[1].x + b.z * xs[2].x;
+    const float a1 = b.x * xs[0].y + b.y * xs[1].y + b.z * xs[2].y;
+    const float a2 = b.x * xs[0].z + b.y * xs[1].z + b.z * xs[2].z;
+    const float C = n.x * (a0 - p.x) + n.y * (a1 - p.y) + n.z * (a2 - p.z);
+    if (C > 0.f) return false;
+    const float bb[3] = {b.x, b.y, b.z};
+    float L = 0.f;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float gx = bb[i] * n.x, gy = bb[i] * n.y, gz = bb[i] * n.z;
+        L += fabsf(xs[i].w) * (gx * gx + gy * gy + gz * gz);
+    }
+    const float dl = -C / L;
+    if (!isfinite(dl)) return false;
+    lam += dl;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float wi = fabsf(xs[i].w);
+        d[i][0] = wi * (bb[i] * n.x) * dl;
+        d[i][1] = wi * (bb[i] * n.y) * dl;
+        d[i][2] = wi * (bb[i] * n.z) * dl;
+    }
+    return true;
+}
+
 // threads of the one-block compaction kernels (rigid contacts, self contacts)
 constexpr int kCompactThreads = 1024;
 

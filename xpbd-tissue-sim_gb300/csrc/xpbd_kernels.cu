@@ -371,38 +371,6 @@ __global__ void __launch_bounds__(kPatchBlock) k_project_patch_reg(TetArrays t, 
 }
 
 
-// Static collision projection of one contact slot: C = n.(u x1 + v x2 + w x3 - p),
-// skipped when C > 0, alpha = 0. Returns false when skipped.
-__device__ __forceinline__ bool contact_update(const ContactArrays& c, int slot, const float4 xs[3], float d[3][3],
-                                               float& lam) {
-    const float4 b = c.bary[slot];
-    const float4 p = c.p[slot];
-    const float4 n = c.n[slot];
-    const float a0 = b.x * xs[0].x + b.y * xs[1].x + b.z * xs[2].x;
-    const float a1 = b.x * xs[0].y + b.y * xs[1].y + b.z * xs[2].y;
-    const float a2 = b.x * xs[0].z + b.y * xs[1].z + b.z * xs[2].z;
-    const float C = n.x * (a0 - p.x) + n.y * (a1 - p.y) + n.z * (a2 - p.z);
-    if (C > 0.f) return false;
-    const float bb[3] = {b.x, b.y, b.z};
-    float L = 0.f;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float gx = bb[i] * n.x, gy = bb[i] * n.y, gz = bb[i] * n.z;
-        L += fabsf(xs[i].w) * (gx * gx + gy * gy + gz * gz);
-    }
-    const float dl = -C / L;
-    if (!isfinite(dl)) return false;
-    lam += dl;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float wi = fabsf(xs[i].w);
-        d[i][0] = wi * (bb[i] * n.x) * dl;
-        d[i][1] = wi * (bb[i] * n.y) * dl;
-        d[i][2] = wi * (bb[i] * n.z) * dl;
-    }
-    return true;
-}
-
 template <bool FIRST>
 __global__ void k_contacts_jacobi(ContactArrays c, const float4* __restrict__ x, float4* __restrict__ dx) {
     pdl_wait_then_release();
@@ -1981,12 +1949,20 @@ int sweep_versioned_blocks_per_sm(int min_blocks, int tasks_per_warp, bool conta
     return n < m ? n : m;
 }
 
+void launch_versions_in(const Launch& s, VerRec* xv, const float4* x, const int* vperm, int V) {
+    go(k_versions_in, nblk(V, 256), 256, s, xv, x, vperm, V);
+}
+
+void launch_versions_out(const Launch& s, float4* x, const VerRec* xv, const int* vperm, int V) {
+    go(k_versions_out, nblk(V, 256), 256, s, x, xv, vperm, V);
+}
+
 cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const PatchArrays& pa, const int4* pver,
                                    const TaskArrays& ta, int iters, bool first_zero, float4* x, VerRec* xv, int V,
                                    const int* vperm, Flags* flags, int grid, int min_blocks, bool resident,
                                    const ContactArrays& ca, const FlowContacts& fc) {
     if (iters <= 0 || ta.ntasks <= 0) return cudaSuccess;
-    go(k_versions_in, nblk(V, 256), 256, s, xv, (const float4*)x, vperm, V);
+    launch_versions_in(s, xv, x, vperm, V);
     const int warps = grid * (kFlowBlock / 32);
     const int per_warp = (ta.ntasks + warps - 1) / warps;
     const bool contacts = fc.task != nullptr;
@@ -2018,7 +1994,7 @@ cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const Pa
 #undef XG_VER_M
 #undef XG_VER
     if (e != cudaSuccess) return e;
-    go(k_versions_out, nblk(V, 256), 256, s, x, (const VerRec*)xv, vperm, V);
+    launch_versions_out(s, x, xv, vperm, V);
     return cudaSuccess;
 }
 

@@ -167,6 +167,55 @@ struct FlowContacts {
 // when the warp owns at most this many tasks per iteration
 constexpr int kResidentTasks = 10;
 
+// Gauss-Seidel on chip (k_sweep_cluster): one thread-block cluster per
+// instance, each block with a run of the instance's patches in mesh order, its
+// vertices, multipliers and patch topology in shared memory.
+constexpr int kClusterLanes = 128;       // patches of one colour a block projects at once: one warp per scheduler
+constexpr int kClusterThreads = 256;     // most threads of a block
+constexpr int kMaxClusterSize = 16;      // blocks of a cluster (above 8: opt-in)
+constexpr unsigned kClusterPolls = 1u << 20;  // polls of a shared vertex before a wait gives up
+constexpr int kMaxClusterColours = 64;   // patch colours, as build_cluster splits them
+constexpr int kClusterSmemMax = 230400;  // dynamic shared memory of a block (227 KB less the static part)
+struct ClusterArrays {
+    const int4* part;       // [2 ncta] (first entry of verts, vertices, of these held by other blocks too,
+                            //  first entry of vidx / meta / ver / slot), (patches, first entry of remote, tets,
+                            //  first tet of rec)
+    const int4* range;      // [ncta ncol] (first patch in the block, patches, tets, first tet in the block)
+    const int4* vidx;       // [P] by block, colour, patch: the patch's vertices, 8 x 16-bit block-local indices
+    const int4* meta;       // [P] first tet in the block, ntets | nverts << 8, layout word
+    const int4* ver;        // [P] per vertex slot 16 bits: patches around the vertex << 8 | those of a lower colour
+    const int* slot;        // [P] first slot
+    const float4* rec;      // [3][nrec] the tet records m0, m1, m2 by block, colour, patch
+    size_t nrec;
+    const int* verts;       // block-local vertex -> vertex, sign bit set in the block that writes it back
+    const uint4* remote;    // the shared vertices' other copies, 8 x 16 bits: block in the cluster << 12 |
+                            // local index, 0xffff = none
+    const uint2* send;      // by block and colour: the shared vertices the colour writes and where to: (local index
+                            // << 16 | block in the cluster << 12 | index there, the vertex's 16 bits of ver)
+    const int* send_off;    // [ncta (ncol + 1)] its ranges
+    const int4* faces;      // [F] block-local vertices of a face in the block that projects its contacts, and
+                            // the patches around each, 8 bits a vertex
+    const int* act_faces;   // after a detection: faces with an active static contact by block and face colour
+    const int* act_off;     // [ncta (nfcol + 1)] its ranges
+};
+struct ClusterShape {
+    int ncta, csize, threads, ncol, nfcol;
+    int max_nv, max_nb, max_p, max_t, max_send;  // largest block: vertices, shared ones, patches, tets, sends
+    int rec_cap;                       // tet records of one staging buffer
+    int resident;                      // 1: every record stays in shared memory; 0: two buffers, one colour each
+    size_t smem;
+};
+struct ClusterIo {
+    float4 *x, *prev, *vel;
+    const float* gdz;   // first order: the inertial z move (else nullptr)
+    VerRec* xv;         // positions from and to these records instead of x (nullptr: x)
+    const int* vperm;
+    float dt, dz;
+    int predict;        // the inertial move (prev <- x first)
+    int finalize;       // fixed vertices back to their position before the substep, and with write_vel v
+    int write_vel;
+};
+
 // Self-collisions (DeformableDeformableCollisionConstraint): a uniform grid
 // over the positions, each tet in the cell of its centroid, queries over the
 // 27 cells around a point; tets larger than a cell in some axis go to an
@@ -297,6 +346,16 @@ cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const Pa
 // needs when each warp owns `tasks_per_warp` tasks (0: not resident), with or
 // without the contact phases
 int sweep_versioned_blocks_per_sm(int min_blocks, int tasks_per_warp, bool contacts);
+// the sweep's vertex records from and to the positions
+void launch_versions_in(const Launch& s, VerRec* xv, const float4* x, const int* vperm, int V);
+void launch_versions_out(const Launch& s, float4* x, const VerRec* xv, const int* vperm, int V);
+// Gauss-Seidel on chip: positions in, iters sweeps (with contacts: each
+// followed by the static contacts), positions and multipliers out, in one launch
+cudaError_t launch_sweep_cluster(const Launch& s, const ClusterArrays& a, const ClusterShape& sh, const TetArrays& t,
+                                 const ClusterIo& io, int iters, bool first_zero, bool separate, bool contacts,
+                                 const ContactArrays& ca, Flags* flags);
+// clusters of this shape that fit the device at once (0: it cannot run)
+int sweep_cluster_fits(const ClusterShape& sh, bool separate, bool contacts);
 // After a detection (the per-instance active lists built): the sweep's
 // contact tables. vface_off/vface/fcol/vdegp are static: per vertex its
 // surface faces (CSR) and patch count, per face its colour.
