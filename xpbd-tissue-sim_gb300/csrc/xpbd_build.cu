@@ -140,16 +140,27 @@ void release(xpbd_ctx* c) {
     c->stream = nullptr;
 }
 
-// Dataflow tasks: runs of up to kTaskPatches consecutive patches of one colour
+// Dataflow tasks: up to kTaskPatches consecutive patches of one colour
 // (tasks therefore in colour order), and for each task the tasks sharing a
 // vertex with it, flagged when theirs is the higher colour.
 int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector<int4>& pverts) {
     const int P = (int)pmeta.size(), V = c->V;
     std::vector<int4> tasks;
     std::vector<int> tcol, task_of(P);
+    // Every colour in as many tasks as the largest one needs, each with an equal
+    // share of its patches (both follow the mesh order): the k-th tasks of the
+    // colours then cover the same part of the mesh, also where the colours
+    // differ in size, and a warp mostly waits for its own earlier tasks. (With
+    // runs of 32 the k-th tasks drift apart: per colour of a sweep 3.95 against
+    // 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47 x 49 x 45, the
+    // same for 48 x 48 x 48.)
+    int per_colour = 1;
     for (int col = 0; col < c->n_tet_colours; col++)
-        for (int q = c->pcol_off[col]; q < c->pcol_off[col + 1]; q += kTaskPatches) {
-            const int n = std::min(kTaskPatches, c->pcol_off[col + 1] - q);
+        per_colour = std::max(per_colour, (c->pcol_off[col + 1] - c->pcol_off[col] + kTaskPatches - 1) / kTaskPatches);
+    for (int col = 0; col < c->n_tet_colours; col++) {
+        const long long first = c->pcol_off[col], count = c->pcol_off[col + 1] - first;
+        for (int i = 0; i < per_colour; i++) {
+            const int q = (int)(first + count * i / per_colour), n = (int)(first + count * (i + 1) / per_colour) - q;
             int slots = 0;
             for (int k = 0; k < n; k++) {
                 task_of[q + k] = (int)tasks.size();
@@ -158,9 +169,10 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
                     return fail(c, XPBD_ERR_STATE, "dataflow: patch %d does not continue its task's slots", q + k);
                 slots += pmeta[q + k].y & 0xff;
             }
-            tasks.push_back(make_int4(q, n, pmeta[q].x, slots));
+            tasks.push_back(n ? make_int4(q, n, pmeta[q].x, slots) : make_int4(0, 0, 0, 0));
             tcol.push_back(col);
         }
+    }
     const int NT = (int)tasks.size();
     auto pv = [&](int q, int k) {
         const int4& a = pverts[2 * (size_t)q + (k >> 2)];
