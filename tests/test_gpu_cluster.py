@@ -156,3 +156,32 @@ def test_on_chip_batch_equals_versioned_batch(lib):
         s.close()
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n", [3, 23, 24])
+def test_residual_and_energy_sums_at_both_tets_per_thread(lib, n):
+    """Below and above the size from which a thread adds up four tets (65,536;
+    a last block that is partly empty): the residual's norm against the sum of
+    the per-constraint residuals it also writes, and the strain energy against
+    FP64 numpy from the same positions, within the FP32 rounding of the terms."""
+    s, X = _solver((n, n, n), num_iters=2, residual_policy=G.RESIDUAL_EVERY_SUBSTEP)
+    s.step(1)
+    r = s.constraint_residual()
+    a, _ = s.residual()
+    hist = s.residual_history()[-1]
+    # every term rounds once to FP32 (2^-24 relative) in the per-constraint vector
+    assert abs(hist - np.sqrt((r * r).sum())) <= 2 ** -23 * hist
+    assert a > 0 and abs(s.residual_noalloc() - a) <= 1e-13 * a
+    x = s.positions()
+    tets, E = s._meshes[0].tets, s._meshes[0].E
+    D0 = (X[tets[:, :3]] - X[tets[:, 3:]]).transpose(0, 2, 1)
+    F = (x[tets[:, :3]] - x[tets[:, 3:]]).transpose(0, 2, 1) @ np.linalg.inv(D0)
+    vol = np.abs(np.linalg.det(D0)) / 6
+    mu, la = E / 2.9, E * 0.45 / (1.45 * 0.1)
+    J = np.linalg.det(F)
+    d = J - 1
+    Ch = np.where(J >= 1, np.log(np.maximum(J, 1)), d - d * d / 2 + d ** 3 / 3) - mu / la
+    ref = (mu * vol * (F * F).sum((1, 2)) + la * vol * Ch * Ch).sum()
+    # FP32 positions (1e-2 m edges in a 0.24 m mesh): F to 3e-6, the energy to twice that
+    assert abs(s.strain_energy() - ref) <= 2e-5 * abs(ref)
+    s.close()

@@ -1441,7 +1441,7 @@ int xpbd_get_lambda(xpbd_ctx* c, double* lam) {
 
 int xpbd_total_strain_energy(xpbd_ctx* c, double* e) {
     if (!c || !e) return XPBD_ERR_INVALID;
-    const int nb = residual_blocks(c->T, c->block);
+    const int nb = residual_grid(c->T, c->block);
     launch_residual(c->L(), c->block, c->tets(), c->T, c->x.p, c->prm.constraint_type == XPBD_CONSTRAINT_SEPARATE,
                     c->perm.p, nullptr, no_sink(), c->energy_partial.p, (float)(c->prm.dt * c->prm.dt));
     launch_reduce_rows(c->L(), c->energy_partial.p, 1, nb, c->energy_partial.p + nb);

@@ -422,6 +422,9 @@ void launch_warm_start(const Launch& s, const TetArrays& t, int T, const float* 
 void launch_warm_fallback(const Launch& s, const double* rows, float4* x, const float4* x_pred, float2* lam, int V,
                           int T, unsigned long long* stats);
 void launch_reduce_rows(const Launch& s, const double* partial, int rows, int stride, double* out);
+// room for a row of residual partials (any kernel that writes one), and the
+// blocks that launch_residual uses of it
 int residual_blocks(int T, int block);
+int residual_grid(int T, int block);
 
 }  // namespace xg
