@@ -212,6 +212,22 @@ bool use_cluster(const xpbd_ctx* c) {
 // part of what the interface reports (xpbd_launch_count).
 bool cluster_fused(const xpbd_ctx* c) { return c->F > 0 || !c->flow_versioned || c->flow_grid > 1; }
 
+// One sweep over the tets between launches that need the positions (contacts,
+// attachments, the residual of every iteration) in one launch on chip, for
+// meshes of one block; false where the colour launches are to run. Per
+// iteration with its residual, GB300: 14.0 against 18.8 us (30 hexes), 19.9
+// against 24.8 us (1,000); from two blocks on a launch of its own for each
+// sweep gains nothing (25-28 against 25-27 us), nor does the versioned sweep
+// (42 against 44 us at 64,000 hexes, 82 against 76 us at 262,144).
+bool enqueue_one_sweep(xpbd_ctx* c, bool first_zero) {
+    if (!c->cluster_on || c->cl_shape.csize > 1 || c->stalled) return false;
+    Scope sc(c, K_PROJECT_GS);
+    const xg::ClusterIo io{c->x.p, c->prev.p, c->vel.p, nullptr, nullptr, nullptr, (float)c->prm.dt, 0.f, 0, 0, 0};
+    launch_sweep_cluster(c->L(), c->cl, c->cl_shape, c->tets(), io, 1, first_zero,
+                         c->prm.constraint_type == XPBD_CONSTRAINT_SEPARATE, false, c->contacts(), c->flags.p);
+    return true;
+}
+
 // solve_only: XPBDSolver::solve() alone (XPBDSolver.hpp:66-97) -- lambda <- 0
 // and num_iters sweeps on the current positions, with no inertial move, no
 // local collision passes, no fixed reset and no rigid-body update.
@@ -368,17 +384,20 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
         for (int it = 0; it < iters; it++) {
             const bool first = it == 0;
             if (every_iter && !(warm && it == 0)) exact_residual_row(c, it, false);
-            const int passes = separate ? 2 : 1;
-            for (int pass = 0; pass < passes; pass++) {
-                const int which = separate ? pass : 2;
-                // in the separate form the second pass (Hyd) of iteration 0
-                // must not re-zero the Dev multipliers updated by pass 0
-                const bool f = first && !warm && (!separate || pass == 0);
-                for (int col = 0; col < c->n_tet_colours; col++) {
-                    Scope sc(c, K_PROJECT_GS);
-                    launch_project_patches(c->L(), c->tets(), c->patches(), c->pcol_off[col], c->pcol_off[col + 1],
-                                           c->x.p, f, which, c->flags.p, c->prm.gs_min_blocks ? c->prm.gs_min_blocks : 6,
-                                           patch_kernel_variant(c->prm.gs_variant));
+            if (!enqueue_one_sweep(c, first && !warm)) {
+                const int passes = separate ? 2 : 1;
+                for (int pass = 0; pass < passes; pass++) {
+                    const int which = separate ? pass : 2;
+                    // in the separate form the second pass (Hyd) of iteration 0
+                    // must not re-zero the Dev multipliers updated by pass 0
+                    const bool f = first && !warm && (!separate || pass == 0);
+                    for (int col = 0; col < c->n_tet_colours; col++) {
+                        Scope sc(c, K_PROJECT_GS);
+                        launch_project_patches(c->L(), c->tets(), c->patches(), c->pcol_off[col], c->pcol_off[col + 1],
+                                               c->x.p, f, which, c->flags.p,
+                                               c->prm.gs_min_blocks ? c->prm.gs_min_blocks : 6,
+                                               patch_kernel_variant(c->prm.gs_variant));
+                    }
                 }
             }
             if (have_faces) {
