@@ -118,7 +118,7 @@ void release(xpbd_ctx* c) {
     c->s_lam.release(); c->s_surf.release(); c->s_cell_count.release(); c->s_cell_off.release();
     c->s_cell_fill.release(); c->s_cell_tets.release(); c->s_tet_cell.release(); c->s_overflow.release();
     c->s_n_overflow.release(); c->s_hit_tet.release(); c->s_hit_list.release(); c->s_n_hits.release();
-    c->s_scan_part.release();
+    c->s_scan_part.release(); c->s_plan.release(); c->s_plan_ids.release();
     c->patch_meta.release(); c->patch_verts.release();
     c->local_slots.release(); c->vmask.release(); c->tmask.release(); c->gdz.release();
     c->d_att_v.release(); c->d_att_order.release(); c->d_att_target.release(); c->d_att_lam.release();
@@ -589,7 +589,8 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
     const double other = separate ? 2.9 : 2.2;
     const int n_min = (int)std::min<size_t>(kMaxClusterSize, (largest + kClusterLanes * ncol - 1) / (kClusterLanes * ncol));
     for (int n : {n_min, n_min + 1, n_min + 2, n_min + 4, kMaxClusterSize}) {
-        if (n > kMaxClusterSize || (K > 1 && K * n > sms) || (!choices.empty() && choices.back().n == n)) continue;
+        // self-collisions take their own launches between the sweeps: one block only
+        if (n > kMaxClusterSize || (n > 1 && c->prm.self_collisions) || (K > 1 && K * n > sms) || (!choices.empty() && choices.back().n == n)) continue;
         for (int sh = 0; sh < 4; sh++) {
             if ((n == 1 && sh > 0) || (sh == 3 && (n & (n - 1)))) continue;
             assign(sh, n);
@@ -947,6 +948,12 @@ int build_self_collisions(xpbd_ctx* c, const std::vector<double>& X, const std::
     XPBD_CU(c, c->s_contact.alloc(ns));
     XPBD_CU(c, c->s_lam.alloc(ns));
     XPBD_CU(c, c->s_scan_part.alloc(c->ncells / 4096 + 2));
+    if (c->prm.solver_type == XPBD_SOLVER_GAUSS_SEIDEL) {
+        XPBD_CU(c, self_prepare_kernels());
+        XPBD_CU(c, c->s_plan.alloc(2 * (size_t)c->n_surf + 3 + V));
+        XPBD_CU(c, c->s_plan_ids.alloc(ns));
+        XPBD_CU(c, cudaMemset(c->n_rounds(), 0, sizeof(int)));
+    }
     XPBD_CU(c, cudaMemcpy(c->s_tets.p, tt.data(), sizeof(int4) * T, cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->s_Q.p, Q.data(), sizeof(double) * 9 * (size_t)T, cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->s_X0.p, X.data(), sizeof(double) * 3 * (size_t)V, cudaMemcpyHostToDevice));

@@ -203,7 +203,7 @@ float self_alpha_tilde(const xpbd_ctx* c) {
 bool use_cluster(const xpbd_ctx* c) {
     return c->cluster_on && !c->lat_on && !c->stalled && c->prm.num_iters > 0 &&
            c->prm.residual_policy != XPBD_RESIDUAL_EVERY_ITERATION && c->att_v.empty() && !c->self_on && !c->nbodies &&
-           (!c->F || c->cluster_contacts);
+           (!c->F || c->cluster_contacts || !c->static_seen);
 }
 
 // A mesh whose largest colour is at most one warp of patches keeps the inertial
@@ -241,7 +241,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     const float dz = (float)(-p.g_accel * p.dt * p.dt);
     cudaStream_t s = c->stream;
     const ContactArrays ca = c->contacts();
-    const bool have_faces = c->F > 0;
+    const bool have_faces = c->F > 0, have_static = have_faces && c->static_seen;
     const bool warm = c->warm_mode != XPBD_WARM_NONE;
     const bool cluster = use_cluster(c);
     // on chip the inertial move is part of the sweep's launch when nothing
@@ -284,7 +284,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
                     launch_project_jacobi_gather_write(c->L(), c->block, c->tets(), c->T, c->x.p, c->dxt.p, first,
                                                        separate, rs, c->flags.p);
                 }
-                if (have_faces) {
+                if (have_static) {
                     Scope sc(c, K_CONTACT);
                     launch_contacts_jacobi(c->L(), ca, c->x.p, c->dx.p, first_contact);
                 }
@@ -312,7 +312,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
                     launch_project_jacobi(c->L(), c->block, c->tets(), c->T, c->x.p, c->dx.p, first, separate, rs,
                                           c->flags.p);
                 }
-                if (have_faces) {
+                if (have_static) {
                     Scope sc(c, K_CONTACT);
                     launch_contacts_jacobi(c->L(), ca, c->x.p, c->dx.p, first_contact);
                 }
@@ -347,7 +347,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
             const xg::ClusterIo io{c->x.p, c->prev.p, c->vel.p, p.first_order ? c->gdz.p : nullptr,
                                    records ? c->xv.p : nullptr, c->vperm.p, dt, dz, fuse_predict, final_on_chip,
                                    write_vel};
-            launch_sweep_cluster(c->L(), c->cl, c->cl_shape, c->tets(), io, iters, !warm, separate, have_faces, ca,
+            launch_sweep_cluster(c->L(), c->cl, c->cl_shape, c->tets(), io, iters, !warm, separate, have_static, ca,
                                  c->flags.p);
         }
         if (records) {
@@ -371,7 +371,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
         Scope sc(c, K_PROJECT_GS);
         if (versioned) {
             const xg::FlowContacts fc =
-                have_faces ? c->flowc() : xg::FlowContacts{nullptr, nullptr, nullptr, nullptr, nullptr};
+                have_static ? c->flowc() : xg::FlowContacts{nullptr, nullptr, nullptr, nullptr, nullptr};
             launch_sweep_versioned(c->L(), c->tets(), c->patches_v(), c->patch_ver.p, c->tasks(), iters, !warm, c->x.p,
                                    c->xv.p, c->V, c->vperm.p, c->flags.p, c->flow_grid, p.gs_min_blocks,
                                    c->flow_resident, ca, fc);
@@ -400,7 +400,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
                     }
                 }
             }
-            if (have_faces) {
+            if (have_static) {
                 Scope sc(c, K_CONTACT);
                 launch_contacts_gs_lists(c->L(), ca, c->act_faces.p, c->act_off.p, c->n_face_colours, c->n_inst,
                                          c->x.p, first);
@@ -513,19 +513,19 @@ int prepare_update(xpbd_ctx* c) {
     // the faces with active static contacts, after the contacts changed, in the
     // form that the coming substep reads
     const bool cluster = use_cluster(c);
-    if (c->F && cluster && c->cluster_lists_dirty) {
+    if (c->static_seen && cluster && c->cluster_lists_dirty) {
         Scope sc(c, K_DETECT);
         launch_contact_lists(c->L(), c->contacts(), c->cl_ifl.p, c->cl_ifo.p, c->n_face_colours, c->cl_shape.ncta,
                              c->cl_act_faces.p, c->cl_act_off.p);
         c->cluster_lists_dirty = false;
     }
-    if (c->F && (!cluster || c->local_slots.p) && c->contact_lists_dirty) {
+    if (c->static_seen && (!cluster || c->local_slots.p) && c->contact_lists_dirty) {
         Scope sc(c, K_DETECT);
         launch_contact_lists(c->L(), c->contacts(), c->ifl.p, c->ifo_off.p, c->n_face_colours, c->n_inst,
                              c->act_faces.p, c->act_off.p);
         c->contact_lists_dirty = false;
     }
-    if (c->flow_contacts && !cluster && c->flow_tables_dirty) {
+    if (c->flow_contacts && c->static_seen && !cluster && c->flow_tables_dirty) {
         Scope sc(c, K_DETECT);
         launch_flow_contact_tables(c->L(), c->contacts(), c->act_faces.p, c->act_off.p, c->n_face_colours, c->n_inst,
                                    c->vface_off.p, c->vface.p, c->fcol_d.p, c->vdeg_p.p, c->factive.p, c->cm_off.p,
@@ -613,9 +613,14 @@ int detect(xpbd_ctx* c) {
         if (st) return st;
         if (c->self_on) {
             Scope sc(c, K_DETECT);
-            launch_self_detect(c->L(), c->selfs(), c->sgrid, c->x.p, c->faces.p);
+            launch_self_detect(c->L(), c->selfs(), c->sgrid, c->x.p, c->faces.p,
+                               c->prm.solver_type == XPBD_SOLVER_JACOBI);
         }
         return after_launches(c, "detect");
+    }
+    if (!c->static_seen) {
+        c->static_seen = true;
+        c->graph_dirty = true;  // the contact phases enter the substep
     }
     if (c->sphere_dirty) {
         // pageable source: the copy is staged before the call returns, so the
@@ -640,7 +645,8 @@ int detect(xpbd_ctx* c) {
     // self-collision tests run after the object pairs (CollisionScene.cpp:44-50)
     if (c->self_on) {
         Scope sc(c, K_DETECT);
-        launch_self_detect(c->L(), c->selfs(), c->sgrid, c->x.p, c->faces.p);
+        launch_self_detect(c->L(), c->selfs(), c->sgrid, c->x.p, c->faces.p,
+                               c->prm.solver_type == XPBD_SOLVER_JACOBI);
     }
     std::fill(c->api_slots.begin(), c->api_slots.end(), -1);  // unknown until read back
     c->contacts_changed();
@@ -1164,6 +1170,7 @@ int xpbd_clear_collisions(xpbd_ctx* c) {
         XPBD_CU(c, cudaMemsetAsync(c->c_lam.p, 0, sizeof(float) * (size_t)c->S * c->F, c->stream));
         XPBD_CU(c, cudaMemsetAsync(c->rc_count.p, 0, sizeof(int), c->stream));
         if (c->self_on) XPBD_CU(c, cudaMemsetAsync(c->s_n_hits.p, 0, sizeof(int), c->stream));
+        if (c->n_rounds()) XPBD_CU(c, cudaMemsetAsync(c->n_rounds(), 0, sizeof(int), c->stream));
         c->contacts_changed();
     }
     std::fill(c->api_slots.begin(), c->api_slots.end(), 0);
@@ -1204,6 +1211,10 @@ int xpbd_add_static_collision(xpbd_ctx* c, int32_t face, double u, double v, dou
     XPBD_CU(c, cudaMemcpy(c->c_lam.p + slot, &z, sizeof z, cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->c_bary.p + slot, &b, sizeof b, cudaMemcpyHostToDevice));
     c->api_slots[face] = s + 1;
+    if (!c->static_seen) {
+        c->static_seen = true;
+        c->graph_dirty = true;
+    }
     c->contacts_changed();
     return XPBD_OK;
 }

@@ -148,6 +148,9 @@ struct xpbd_ctx {
     // static contacts by instance and face colour: all faces (ifl, ifo_off) and,
     // after each detection, those with an active contact (act_faces, act_off)
     DevBuf<int> ifl, ifo_off, act_faces, act_off;
+    // a static contact has been detected or added once: before, the contact
+    // arrays are empty and the substep leaves their phases out
+    bool static_seen = false;
     // out of date after a detection: the per-instance lists, the versioned
     // sweep's tables and the on-chip sweep's lists (each built when a route uses it)
     bool contact_lists_dirty = true, flow_tables_dirty = true, cluster_lists_dirty = true;
@@ -162,7 +165,8 @@ struct xpbd_ctx {
     DevBuf<float4> s_X0f;
     DevBuf<float> s_lam;
     DevBuf<int> s_surf, s_cell_count, s_cell_off, s_cell_fill, s_cell_tets, s_tet_cell, s_overflow, s_n_overflow,
-        s_hit_tet, s_hit_list, s_n_hits, s_scan_part;
+        s_hit_tet, s_hit_list, s_n_hits, s_scan_part, s_plan;
+    DevBuf<int4> s_plan_ids;
     DevBuf<int> face_inst;
     bool sphere_dirty = true;
     int n_spheres_total = 0;
@@ -231,12 +235,14 @@ struct xpbd_ctx {
     xg::FlowContacts flowc() {
         return xg::FlowContacts{ctask.p, cface.p, n_ctasks.p, vdeg_c.p, faces_v.p};
     }
+    int* n_rounds() { return s_plan.p ? s_plan.p + 2 * n_surf + 2 : nullptr; }  // in s_plan: plan, round_off, this, owner
     xg::SelfArrays selfs() {
         return xg::SelfArrays{s_tets.p,        s_Q.p,          s_X0.p,         s_X0f.p,      s_surf.p,
                               n_surf,          s_cell_count.p, s_cell_off.p,   s_cell_fill.p, s_cell_tets.p,
                               s_tet_cell.p,    s_overflow.p,   s_n_overflow.p, s_hit_tet.p,  s_hit_list.p,
                               s_n_hits.p,      s_contact.p,    s_lam.p,        s_scan_part.p, T,
-                              F};
+                              F,               s_plan.p,       s_plan_ids.p,   s_plan.p ? s_plan.p + n_surf : nullptr,
+                              n_rounds(),      s_plan.p ? s_plan.p + 2 * n_surf + 3 : nullptr, V};
     }
     TetArrays tets() {
         return TetArrays{tet_idx.p, m0.p, m1.p, m2.p, lam.p, q0.p, q1.p, q2.p};

@@ -245,6 +245,13 @@ struct SelfArrays {
     float* lam;             // [n_surf]
     int* scan_part;         // scan scratch, [ncells / 4096 + 2]
     int T, F;
+    // Gauss-Seidel: the contacts in rounds that share no vertex (k_self_plan)
+    int* plan;              // [n_surf] contacts, round by round
+    int4* plan_ids;         // [n_surf] their vertices
+    int* round_off;         // [n_surf + 2] the rounds' ranges
+    int* n_rounds;          // [1] -1: too many contacts, in detection order instead
+    int* owner;             // [V] scratch
+    int V;
 };
 
 struct Flags {
@@ -396,7 +403,9 @@ void launch_rigid_contacts(const Launch& s, const ContactArrays& c, const int* l
 void launch_rigid_update(const Launch& s, double* rb, int nb, double dt, double g);
 void launch_rigid_velocity(const Launch& s, double* rb, int nb, double dt);
 // self-collision detection (after the SDF contacts) and projection
-void launch_self_detect(const Launch& s, const SelfArrays& a, const SelfGrid& g, const float4* x, const int4* faces);
+void launch_self_detect(const Launch& s, const SelfArrays& a, const SelfGrid& g, const float4* x, const int4* faces,
+                        bool jacobi);
+cudaError_t self_prepare_kernels();
 void launch_self_contacts(const Launch& s, const SelfArrays& a, const int4* faces, float4* x, float4* dx,
                           bool jacobi, bool first, float alpha_tilde, Flags* flags);
 // positions and velocities from / to host arrays the device can address

@@ -157,10 +157,14 @@ __device__ __forceinline__ bool same_side_f(const float* p, const float* a, cons
 }
 
 // EmbreeScene::tetMeshSelfCollisionQuery: the lowest-index tet holding the
-// surface vertex among those that do not have it as a vertex
-__global__ void k_self_query(SelfArrays a, SelfGrid g, const float4* __restrict__ x) {
+// surface vertex among those that do not have it as a vertex. One warp a
+// vertex: the 27 cells are nine runs of up to three neighbours in the sorted
+// tet list, whose tets the lanes test 32 at a time (a chain of three dependent
+// loads each; one thread a vertex walked about 150 of them, 129 us for 1,734
+// vertices, now 10).
+__global__ void __launch_bounds__(128) k_self_query(SelfArrays a, SelfGrid g, const float4* __restrict__ x) {
     pdl_wait_then_release();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= a.n_surf) return;
     const int v = a.surf[k];
     const float4 pv = x[v];
@@ -179,15 +183,35 @@ __global__ void k_self_query(SelfArrays a, SelfGrid g, const float4* __restrict_
     };
     const int cx = grid_cell1(p[0], g.ox, g.cell, g.nx), cy = grid_cell1(p[1], g.oy, g.cell, g.ny),
               cz = grid_cell1(p[2], g.oz, g.cell, g.nz);
-    for (int z = max(cz - 1, 0); z <= min(cz + 1, g.nz - 1); z++)
-        for (int y = max(cy - 1, 0); y <= min(cy + 1, g.ny - 1); y++)
-            for (int xx = max(cx - 1, 0); xx <= min(cx + 1, g.nx - 1); xx++) {
-                const int c = (z * g.ny + y) * g.nx + xx;
-                for (int i = a.cell_off[c]; i < a.cell_off[c + 1]; i++) test(a.cell_tets[i]);
-            }
+    // lane r < 9: the run of cells (cx - 1 .. cx + 1) of row r
+    int from = 0, len = 0;
+    if (lane < 9) {
+        const int y = cy + lane % 3 - 1, z = cz + lane / 3 - 1;
+        if (y >= 0 && y < g.ny && z >= 0 && z < g.nz) {
+            const int row = (z * g.ny + y) * g.nx;
+            from = a.cell_off[row + max(cx - 1, 0)];
+            len = a.cell_off[row + min(cx + 1, g.nx - 1) + 1] - from;
+        }
+    }
+    int end[9], start[9], total = 0;
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const int n = __shfl_sync(0xffffffffu, len, r);
+        start[r] = __shfl_sync(0xffffffffu, from, r) - total;
+        total += n;
+        end[r] = total;
+    }
+    for (int i = lane; i < total; i += 32) {
+        int at = start[0];
+#pragma unroll
+        for (int r = 1; r < 9; r++)
+            if (i >= end[r - 1]) at = start[r];
+        test(a.cell_tets[at + i]);
+    }
     const int no = *a.n_overflow;
-    for (int i = 0; i < no; i++) test(a.overflow[i]);
-    a.hit_tet[k] = best == INT_MAX ? -1 : best;
+    for (int i = lane; i < no; i += 32) test(a.overflow[i]);
+    best = __reduce_min_sync(0xffffffffu, best);
+    if (lane == 0) a.hit_tet[k] = best == INT_MAX ? -1 : best;
 }
 
 // the surface indices with a hit, ascending (one block)
@@ -261,16 +285,9 @@ __device__ float point_triangle_distance_f(const float* p, const float* a, const
     return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1)), __fmul_rn(e2, e2)));
 }
 
-// DeformableMeshSDF::closestSurfaceFaceToPointInTet (DeformableMeshSDF.cpp:68-82),
-// one warp per hit: the vertex mapped to rest space through the tet it is in
-// (F = Ds Dm^-1 in double, none when |det F| < 1e-8), then the closest face of
-// the rest surface (float; of equally close faces the lowest index)
-__global__ void k_self_face(SelfArrays a, const float4* __restrict__ x, const int4* __restrict__ faces) {
-    pdl_wait_then_release();
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= *a.n_hits) return;
-    const int k = a.hit_list[w];
-    const int v = a.surf[k], t = a.hit_tet[k];
+// the surface vertex v mapped to rest space through tet t into pm; 0 when the
+// tet is degenerate
+__device__ int rest_point(const SelfArrays& a, const float4* __restrict__ x, int v, int t, float* pm) {
     const int4 e = a.tets[t];
     const int ids[5] = {e.x, e.y, e.z, e.w, v};
     double xd[5][3];
@@ -290,47 +307,80 @@ __global__ void k_self_face(SelfArrays a, const float4* __restrict__ x, const in
     const double c10 = M(1, 2) * M(2, 0) - M(1, 0) * M(2, 2);
     const double c20 = M(1, 0) * M(2, 1) - M(1, 1) * M(2, 0);
     const double det = M(0, 0) * c00 + M(0, 1) * c10 + M(0, 2) * c20;
-    int face = -1;
-    if (!(fabs(det) < 1e-8)) {
-        const double inv = 1.0 / det;
-        double Fi[9];
-        Fi[0] = c00 * inv; Fi[1] = c10 * inv; Fi[2] = c20 * inv;
-        Fi[3] = (M(0, 2) * M(2, 1) - M(0, 1) * M(2, 2)) * inv;
-        Fi[4] = (M(0, 0) * M(2, 2) - M(0, 2) * M(2, 0)) * inv;
-        Fi[5] = (M(0, 1) * M(2, 0) - M(0, 0) * M(2, 1)) * inv;
-        Fi[6] = (M(0, 1) * M(1, 2) - M(0, 2) * M(1, 1)) * inv;
-        Fi[7] = (M(0, 2) * M(1, 0) - M(0, 0) * M(1, 2)) * inv;
-        Fi[8] = (M(0, 0) * M(1, 1) - M(0, 1) * M(1, 0)) * inv;
-        const double rel[3] = {xd[4][0] - xd[3][0], xd[4][1] - xd[3][1], xd[4][2] - xd[3][2]};
-        float pm[3];
-        for (int r = 0; r < 3; r++)
-            pm[r] = (float)(Fi[r] * rel[0] + Fi[3 + r] * rel[1] + Fi[6 + r] * rel[2] + a.X0[3 * (size_t)e.w + r]);
+    if (fabs(det) < 1e-8) return 0;
+    const double inv = 1.0 / det;
+    double Fi[9];
+    Fi[0] = c00 * inv; Fi[1] = c10 * inv; Fi[2] = c20 * inv;
+    Fi[3] = (M(0, 2) * M(2, 1) - M(0, 1) * M(2, 2)) * inv;
+    Fi[4] = (M(0, 0) * M(2, 2) - M(0, 2) * M(2, 0)) * inv;
+    Fi[5] = (M(0, 1) * M(2, 0) - M(0, 0) * M(2, 1)) * inv;
+    Fi[6] = (M(0, 1) * M(1, 2) - M(0, 2) * M(1, 1)) * inv;
+    Fi[7] = (M(0, 2) * M(1, 0) - M(0, 0) * M(1, 2)) * inv;
+    Fi[8] = (M(0, 0) * M(1, 1) - M(0, 1) * M(1, 0)) * inv;
+    const double rel[3] = {xd[4][0] - xd[3][0], xd[4][1] - xd[3][1], xd[4][2] - xd[3][2]};
+    for (int r = 0; r < 3; r++)
+        pm[r] = (float)(Fi[r] * rel[0] + Fi[3 + r] * rel[1] + Fi[6 + r] * rel[2] + a.X0[3 * (size_t)e.w + r]);
+    return 1;
+}
+
+// DeformableMeshSDF::closestSurfaceFaceToPointInTet (DeformableMeshSDF.cpp:68-82):
+// the vertex mapped to rest space through the tet it is in (F = Ds Dm^-1 in
+// double, none when |det F| < 1e-8), then the closest face of the rest surface
+// (float; of equally close faces the lowest index). One block a hit, one
+// thread its rest point (FP64) and all of them the faces: a warp a hit took
+// 122 us for 3,456 faces, all of it the chain of its own 108 rounds; now 23.
+constexpr int kFaceThreads = 256;
+__global__ void __launch_bounds__(kFaceThreads) k_self_face(SelfArrays a, const float4* __restrict__ x,
+                                                            const int4* __restrict__ faces) {
+    __shared__ float spm[3];
+    __shared__ int sok, sbf[kFaceThreads / 32];
+    __shared__ float sbd[kFaceThreads / 32];
+    pdl_wait_then_release();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n = *a.n_hits;
+    for (int w = blockIdx.x; w < n; w += gridDim.x) {
+        const int v = a.surf[a.hit_list[w]];
+        if (threadIdx.x == 0) sok = rest_point(a, x, v, a.hit_tet[a.hit_list[w]], spm);
+        __syncthreads();
         float bd = INFINITY;
         int bf = INT_MAX;
-        for (int f = lane; f < a.F; f += 32) {
-            const int4 fv = faces[f];
-            const float4 A = a.X0f[fv.x], B = a.X0f[fv.y], Cc = a.X0f[fv.z];
-            const float pa[3] = {A.x, A.y, A.z}, pb[3] = {B.x, B.y, B.z}, pc[3] = {Cc.x, Cc.y, Cc.z};
-            const float d = point_triangle_distance_f(pm, pa, pb, pc);
-            if (d < bd) {
-                bd = d;
-                bf = f;
+        if (sok) {
+            const float pm[3] = {spm[0], spm[1], spm[2]};
+#pragma unroll 2
+            for (int f = threadIdx.x; f < a.F; f += kFaceThreads) {
+                const int4 fv = faces[f];
+                const float4 A = a.X0f[fv.x], B = a.X0f[fv.y], Cc = a.X0f[fv.z];
+                const float qa[3] = {A.x, A.y, A.z}, qb[3] = {B.x, B.y, B.z}, qc[3] = {Cc.x, Cc.y, Cc.z};
+                const float d = point_triangle_distance_f(pm, qa, qb, qc);
+                if (d < bd) {
+                    bd = d;
+                    bf = f;
+                }
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-            const int of = __shfl_xor_sync(0xffffffffu, bf, o);
+        auto closer = [&](float od, int of) {
             if (od < bd || (od == bd && of < bf)) {
                 bd = od;
                 bf = of;
             }
+        };
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float od = __shfl_xor_sync(0xffffffffu, bd, o);
+            const int of = __shfl_xor_sync(0xffffffffu, bf, o);
+            closer(od, of);
         }
-        face = bf == INT_MAX ? -1 : bf;
+        if (lane == 0) {
+            sbd[wid] = bd;
+            sbf[wid] = bf;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < kFaceThreads / 32; i++) closer(sbd[i], sbf[i]);
+            a.contact[w] = make_int2(v, bf == INT_MAX ? -1 : bf);
+        }
+        __syncthreads();
     }
-    if (lane == 0) a.contact[w] = make_int2(v, face);
 }
-
 // DeformableDeformableCollisionConstraint::evaluate / gradient
 // (DeformableDeformableCollisionConstraint.cpp): C = (q - p1).a/|a| + 1e-5,
 // a = (p2 - p1) x (p3 - p1); the gradient as the reference writes it (the
@@ -371,21 +421,18 @@ __device__ float self_contact_eval(const float* q, const float* p1, const float*
 }
 
 // ConstraintProjector::project (ConstraintProjector.hpp:111-172) of self
-// contact j: skipped when C > 0; alpha~ = 1e-8/dt^2 (or /dt)
-__device__ bool self_update(const SelfArrays& a, int j, const int4* __restrict__ faces, const float4* x, bool first,
-                            float at, int ids[4], float4 xs[4], float d[4][3], Flags* flags) {
-    const int2 ct = a.contact[j];
-    if (ct.y < 0) return false;
-    const int4 fv = faces[ct.y];
-    ids[0] = ct.x; ids[1] = fv.x; ids[2] = fv.y; ids[3] = fv.z;
+// contact j on the vertices ids (surface vertex, face): skipped when C > 0;
+// alpha~ = 1e-8/dt^2 (or /dt)
+__device__ bool self_update(const SelfArrays& a, int j, const int4& ids, const float4* x, bool first, float at,
+                            float4 xs[4], float d[4][3], Flags* flags) {
+    float lam = first ? 0.f : a.lam[j];
+    xs[0] = x[ids.x]; xs[1] = x[ids.y]; xs[2] = x[ids.z]; xs[3] = x[ids.w];
     float p[4][3];
     for (int i = 0; i < 4; i++) {
-        xs[i] = x[ids[i]];
         p[i][0] = xs[i].x; p[i][1] = xs[i].y; p[i][2] = xs[i].z;
     }
     float g[12];
     const float C = self_contact_eval(p[0], p[1], p[2], p[3], g);
-    float lam = first ? 0.f : a.lam[j];
     bool ok = false;
     if (!(C > 0.f)) {
         float L = at;
@@ -405,21 +452,171 @@ __device__ bool self_update(const SelfArrays& a, int j, const int4* __restrict__
     return ok;
 }
 
-// Gauss-Seidel: the contacts in detection (vertex) order, one thread
-__global__ void k_self_contacts_gs(SelfArrays a, const int4* __restrict__ faces, float4* __restrict__ x, bool first,
-                                   float at, Flags* flags) {
+__device__ __forceinline__ int4 self_ids(const SelfArrays& a, int j, const int4* __restrict__ faces) {
+    const int2 ct = a.contact[j];
+    if (ct.y < 0) return make_int4(-1, -1, -1, -1);
+    const int4 fv = faces[ct.y];
+    return make_int4(ct.x, fv.x, fv.y, fv.z);
+}
+
+// After a detection: the Gauss-Seidel contacts in rounds that keep the effect
+// of detection order. In each round every contact that is left bids for its
+// four vertices with its number; one that holds all four has no earlier
+// contact left on any of them and goes into the round. Contacts of one round
+// share no vertex, and of two on a common vertex the earlier one is in the
+// earlier round. One block; the bids lie in shared memory, by each vertex's
+// lowest (contact, corner) number, or beyond kPlanShared contacts in owner[].
+// owner is all 0x7f bytes before and after.
+constexpr int kPlanThreads = 1024, kPlanShared = 4096, kPlanMost = 32 * kPlanThreads;
+constexpr int kNoOwner = 0x7f7f7f7f;
+__global__ void __launch_bounds__(kPlanThreads) k_self_plan(SelfArrays a, const int4* __restrict__ faces) {
+    extern __shared__ int bids[];  // [4 kPlanShared] bids, [4 kPlanShared] the vertices' numbers
+    __shared__ int placed, left;
     pdl_wait_then_release();
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const int n = *a.n_hits;
-    for (int j = 0; j < n; j++) {
-        int ids[4];
-        float4 xs[4];
-        float d[4][3];
-        if (!self_update(a, j, faces, x, first, at, ids, xs, d, flags)) continue;
-        for (int i = 0; i < 4; i++) {
-            const float4 c = x[ids[i]];  // a vertex may repeat: add to the current value
-            x[ids[i]] = make_float4(c.x + d[i][0], c.y + d[i][1], c.z + d[i][2], c.w);
+    const int n = *a.n_hits, tid = threadIdx.x;
+    if (n > kPlanMost) {  // more than a thread's 32 bits: the projection walks them one by one
+        if (tid == 0) *a.n_rounds = -1;
+        return;
+    }
+    const bool small = n <= kPlanShared;
+    volatile int* const owner = a.owner;
+    unsigned mine = 0;  // contacts tid + 1024 b that are left
+    if (tid == 0) placed = 0;
+    for (int b = 0; tid + kPlanThreads * b < n; b++) {
+        const int j = tid + kPlanThreads * b;
+        const int4 id = self_ids(a, j, faces);
+        if (id.x < 0) continue;
+        mine |= 1u << b;
+        if (small) {
+            const int v[4] = {id.x, id.y, id.z, id.w};
+            for (int k = 0; k < 4; k++) atomicMin(a.owner + v[k], 4 * j + k);
         }
+    }
+    __syncthreads();
+    if (small) {
+        for (int i = tid; i < 4 * n; i += kPlanThreads) bids[i] = kNoOwner;
+        for (unsigned m = mine; m; m &= m - 1) {
+            const int j = tid + kPlanThreads * (__ffs((int)m) - 1);
+            const int4 id = self_ids(a, j, faces);
+            const int v[4] = {id.x, id.y, id.z, id.w};
+            for (int k = 0; k < 4; k++) bids[4 * kPlanShared + 4 * j + k] = owner[v[k]];
+        }
+        __syncthreads();
+        for (unsigned m = mine; m; m &= m - 1) {
+            const int4 id = self_ids(a, tid + kPlanThreads * (__ffs((int)m) - 1), faces);
+            owner[id.x] = kNoOwner; owner[id.y] = kNoOwner; owner[id.z] = kNoOwner; owner[id.w] = kNoOwner;
+        }
+        __syncthreads();
+    }
+    int round = 0;
+    for (;;) {
+        if (tid == 0) {
+            a.round_off[round] = placed;
+            left = 0;
+        }
+        auto each = [&](unsigned set, auto&& f) {
+            for (unsigned m = set; m; m &= m - 1) {
+                const int b = __ffs((int)m) - 1, j = tid + kPlanThreads * b;
+                int at[4];
+                if (small) {
+                    for (int k = 0; k < 4; k++) at[k] = bids[4 * kPlanShared + 4 * j + k];
+                } else {
+                    const int4 id = self_ids(a, j, faces);
+                    at[0] = id.x; at[1] = id.y; at[2] = id.z; at[3] = id.w;
+                }
+                f(b, j, at);
+            }
+        };
+        volatile int* const own = small ? bids : a.owner;
+        each(mine, [&](int, int j, const int* at) {
+            for (int k = 0; k < 4; k++) atomicMin((int*)own + at[k], j);
+        });
+        __syncthreads();
+        unsigned ready = 0;
+        each(mine, [&](int b, int j, const int* at) {
+            if (own[at[0]] == j && own[at[1]] == j && own[at[2]] == j && own[at[3]] == j) ready |= 1u << b;
+        });
+        __syncthreads();
+        each(ready, [&](int, int j, const int* at) {
+            for (int k = 0; k < 4; k++) own[at[k]] = kNoOwner;
+            const int i = atomicAdd(&placed, 1);
+            a.plan[i] = j;
+            a.plan_ids[i] = self_ids(a, j, faces);
+        });
+        mine &= ~ready;
+        if (mine) left = 1;
+        __syncthreads();
+        round++;
+        if (!left) break;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        a.round_off[round] = placed;
+        *a.n_rounds = round;
+    }
+}
+
+// Gauss-Seidel: the contacts as in detection (vertex) order, by the rounds of
+// k_self_plan, one block. (One thread walking the list took 264 us for two
+// 12^3 cubes in contact, four dependent loads and 0.4 us of arithmetic a
+// contact; the rounds 48 us.)
+constexpr int kSelfGsThreads = 128;
+__device__ __forceinline__ void self_contact_gs(const SelfArrays& a, int j, const int4& ids, float4* __restrict__ x,
+                                                bool first, float at, Flags* flags) {
+    float4 xs[4];
+    float d[4][3];
+    if (!self_update(a, j, ids, x, first, at, xs, d, flags)) return;
+    const int v[4] = {ids.x, ids.y, ids.z, ids.w};
+    if (v[0] != v[1] && v[0] != v[2] && v[0] != v[3] && v[1] != v[2] && v[1] != v[3] && v[2] != v[3]) {
+        for (int i = 0; i < 4; i++)
+            x[v[i]] = make_float4(xs[i].x + d[i][0], xs[i].y + d[i][1], xs[i].z + d[i][2], xs[i].w);
+    } else {
+        for (int i = 0; i < 4; i++) {
+            const float4 c = x[v[i]];  // a vertex may repeat: add to the current value
+            x[v[i]] = make_float4(c.x + d[i][0], c.y + d[i][1], c.z + d[i][2], c.w);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kSelfGsThreads) k_self_contacts_gs(SelfArrays a, const int4* __restrict__ faces,
+                                                                     float4* __restrict__ x, bool first, float at,
+                                                                     Flags* flags) {
+    pdl_wait_then_release();
+    const int rounds = *a.n_rounds;
+    if (rounds < 0) {
+        if (threadIdx.x != 0) return;
+        const int n = *a.n_hits;
+        for (int j = 0; j < n; j++) {
+            const int4 ids = self_ids(a, j, faces);
+            if (ids.x >= 0) self_contact_gs(a, j, ids, x, first, at, flags);
+        }
+        return;
+    }
+    // a round's first contacts are loaded while the one before runs
+    int lo = rounds > 0 ? a.round_off[0] : 0, hi = rounds > 0 ? a.round_off[1] : 0;
+    int i = lo + threadIdx.x, j = 0;
+    int4 ids = make_int4(0, 0, 0, 0);
+    if (i < hi) {
+        j = a.plan[i];
+        ids = a.plan_ids[i];
+    }
+    for (int r = 0; r < rounds; r++) {
+        const int nhi = r + 1 < rounds ? a.round_off[r + 2] : hi;
+        const int ni = hi + threadIdx.x;
+        int nj = 0;
+        int4 nids = make_int4(0, 0, 0, 0);
+        if (r + 1 < rounds && ni < nhi) {
+            nj = a.plan[ni];
+            nids = a.plan_ids[ni];
+        }
+        if (i < hi) self_contact_gs(a, j, ids, x, first, at, flags);
+        for (int k = i + kSelfGsThreads; k < hi; k += kSelfGsThreads)
+            self_contact_gs(a, a.plan[k], a.plan_ids[k], x, first, at, flags);
+        __syncthreads();
+        i = ni;
+        hi = nhi;
+        j = nj;
+        ids = nids;
     }
 }
 
@@ -429,16 +626,18 @@ __global__ void k_self_contacts_jacobi(SelfArrays a, const int4* __restrict__ fa
     pdl_wait_then_release();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= *a.n_hits) return;
-    int ids[4];
+    const int4 ids = self_ids(a, j, faces);
     float4 xs[4];
     float d[4][3];
-    if (!self_update(a, j, faces, x, first, at, ids, xs, d, flags)) return;
-    for (int i = 0; i < 4; i++) add_vec4(dx + ids[i], d[i][0], d[i][1], d[i][2]);
+    if (ids.x < 0 || !self_update(a, j, ids, x, first, at, xs, d, flags)) return;
+    const int v[4] = {ids.x, ids.y, ids.z, ids.w};
+    for (int i = 0; i < 4; i++) add_vec4(dx + v[i], d[i][0], d[i][1], d[i][2]);
 }
 
 }  // namespace
 
-void launch_self_detect(const Launch& s, const SelfArrays& a, const SelfGrid& g, const float4* x, const int4* faces) {
+void launch_self_detect(const Launch& s, const SelfArrays& a, const SelfGrid& g, const float4* x, const int4* faces,
+                        bool jacobi) {
     if (a.n_surf <= 0 || a.T <= 0) return;
     const int ncells = g.nx * g.ny * g.nz;
     cudaMemsetAsync(a.cell_count, 0, sizeof(int) * (size_t)ncells, s.s);
@@ -450,9 +649,22 @@ void launch_self_detect(const Launch& s, const SelfArrays& a, const SelfGrid& g,
     go(k_scan_part_single, 1, kScanThreads, s, a.scan_part, nb);
     go(k_scan_apply, nb, kScanThreads, s, (const int*)a.cell_count, ncells, (const int*)a.scan_part, a.cell_off, nb);
     go(k_self_bin_fill, nblk(a.T, 256), 256, s, a);
-    go(k_self_query, nblk(a.n_surf, 128), 128, s, a, g, x);
+    go(k_self_query, nblk(32 * (long long)a.n_surf, 128), 128, s, a, g, x);
     go(k_self_compact, 1, kCompactThreads, s, a);
-    go(k_self_face, nblk(32 * a.n_surf, 256), 256, s, a, x, faces);
+    go(k_self_face, a.n_surf < 1024 ? a.n_surf : 1024, kFaceThreads, s, a, x, faces);
+    if (!jacobi) {
+        cudaMemsetAsync(a.owner, 0x7f, sizeof(int) * (size_t)a.V, s.s);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(kPlanThreads);
+        cfg.dynamicSmemBytes = 8 * sizeof(int) * kPlanShared;
+        cfg.stream = s.s;
+        cudaLaunchKernelEx(&cfg, k_self_plan, a, faces);
+    }
+}
+
+cudaError_t self_prepare_kernels() {
+    return cudaFuncSetAttribute(k_self_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * sizeof(int) * kPlanShared);
 }
 
 void launch_self_contacts(const Launch& s, const SelfArrays& a, const int4* faces, float4* x, float4* dx,
@@ -460,7 +672,7 @@ void launch_self_contacts(const Launch& s, const SelfArrays& a, const int4* face
     if (a.n_surf <= 0) return;
     if (jacobi) go(k_self_contacts_jacobi, nblk(a.n_surf, 128), 128, s, a, faces, (const float4*)x, dx, first,
                    alpha_tilde, flags);
-    else go(k_self_contacts_gs, 1, 32, s, a, faces, x, first, alpha_tilde, flags);
+    else go(k_self_contacts_gs, 1, kSelfGsThreads, s, a, faces, x, first, alpha_tilde, flags);
 }
 
 }  // namespace xg
