@@ -106,9 +106,9 @@ int greedy_colour(long long n, int arity, const int* items, long long nv, int* o
 void release(xpbd_ctx* c) {
     drop_graphs(c);
     for (auto e : c->prof.pool) cudaEventDestroy(e);
-    c->x.release(); c->prev.release(); c->vel.release(); c->dx.release(); c->dxt.release();
+    c->x.release(); c->prev.release(); c->vel.release(); c->dx.release(); c->jb_tab.release(); c->jb_part.release();
     c->tet_idx.release(); c->q0.release(); c->q1.release(); c->q2.release(); c->m0.release(); c->m1.release(); c->m2.release(); c->lam.release();
-    c->perm.release(); c->csr_off.release(); c->csr_ent.release(); c->faces.release(); c->face_list.release();
+    c->perm.release(); c->faces.release(); c->face_list.release();
     c->c_bary.release(); c->c_p.release(); c->c_n.release(); c->c_lam.release();
     c->kin_idx.release(); c->kin_rest.release(); c->flags.release();
     c->sphere_tab.release(); c->face_inst.release();
@@ -872,6 +872,76 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
     return XPBD_OK;
 }
 
+// Jacobi blocks: runs of up to kJacobiTets consecutive slots on at most
+// kJacobiVerts vertices.
+int build_jacobi_blocks(xpbd_ctx* c, const std::vector<int4>& idx) {
+    const int T = c->T, V = c->V;
+    std::vector<int4> block;
+    std::vector<int> vert, local(V), stamp(V, -1), count;
+    block.reserve(T / kJacobiTets + 1);
+    vert.reserve(T);
+    // the tables lie in one buffer: corners and lists first, written in place
+    const size_t o_list = ((size_t)T + 3) / 4, o_rest = o_list + ((size_t)T + 1) / 2;
+    std::vector<int4> tab(o_rest);
+    unsigned char* corner = (unsigned char*)tab.data();
+    unsigned short* list = (unsigned short*)(tab.data() + o_list);
+    for (int t = 0; t < T;) {
+        const int b = (int)block.size(), v0 = (int)vert.size();
+        int n = 0;
+        for (; n < kJacobiTets && t + n < T; n++) {
+            const int* e = &idx[t + n].x;
+            int fresh = 0;
+            for (int k = 0; k < 4; k++) fresh += stamp[e[k]] != b;
+            if ((int)vert.size() - v0 + fresh > kJacobiVerts) break;
+            for (int k = 0; k < 4; k++) {
+                if (stamp[e[k]] != b) {
+                    stamp[e[k]] = b;
+                    local[e[k]] = (int)vert.size() - v0;
+                    vert.push_back(e[k]);
+                }
+                corner[4 * (size_t)(t + n) + k] = (unsigned char)local[e[k]];
+            }
+        }
+        block.push_back(make_int4(t, n, v0, (int)vert.size() - v0));
+        t += n;
+    }
+    const size_t E = vert.size();
+    std::vector<unsigned> range(E);
+    for (const int4& bk : block) {
+        const unsigned char* l = corner + 4 * (size_t)bk.x;
+        count.assign(bk.w + 1, 0);
+        for (int i = 0; i < 4 * bk.y; i++) count[l[i] + 1]++;
+        for (int v = 0; v < bk.w; v++) {
+            range[bk.z + v] = (unsigned)count[v] << 16 | (unsigned)count[v + 1];
+            count[v + 1] += count[v];
+        }
+        for (int i = 0; i < 4 * bk.y; i++) list[4 * (size_t)bk.x + count[l[i]]++] = (unsigned short)i;
+    }
+    std::vector<int> off(V + 1, 0), ent(E);
+    for (size_t e = 0; e < E; e++) off[vert[e] + 1]++;
+    for (int v = 0; v < V; v++) off[v + 1] += off[v];
+    std::vector<int> fill(off.begin(), off.end() - 1);
+    for (size_t e = 0; e < E; e++) ent[fill[vert[e]]++] = (int)e;
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = tab.size();
+        tab.resize(at + (bytes + 15) / 16);
+        std::memcpy(&tab[at], p, bytes);
+        return at;
+    };
+    tab.reserve(o_rest + block.size() + 3 * (E / 4 + 1) + (size_t)V / 4 + 2);
+    const size_t o_block = put(block.data(), sizeof(int4) * block.size()), o_vert = put(vert.data(), sizeof(int) * E),
+                 o_range = put(range.data(), sizeof(unsigned) * E), o_off = put(off.data(), sizeof(int) * off.size()),
+                 o_ent = put(ent.data(), sizeof(int) * E);
+    XPBD_CU(c, c->jb_tab.alloc(tab.size()));
+    XPBD_CU(c, c->jb_part.alloc(E));
+    XPBD_CU(c, cudaMemcpy(c->jb_tab.p, tab.data(), sizeof(int4) * tab.size(), cudaMemcpyHostToDevice));
+    const int4* d = c->jb_tab.p;
+    c->jb = JacobiBlocks{d + o_block, (const int*)(d + o_vert), (const uchar4*)d,
+                         (const unsigned*)(d + o_range), (const unsigned short*)(d + o_list),
+                         (const int*)(d + o_off), (const int*)(d + o_ent), (int)block.size()};
+    return XPBD_OK;
+}
+
 // Self-collision data: the surface vertices, tets in index order, Dm^-1 and
 // rest positions in double, and a uniform grid over the rest bounding box
 // padded by a quarter of its extent, cells 1.1x the widest tet box at rest
@@ -1223,22 +1293,6 @@ int build(xpbd_ctx* c, const xpbd_mesh_desc* ms, int n_inst) {
         }
     }
 
-    // CSR vertex -> (slot, local vertex) for the gather variant
-    std::vector<int> off(V + 1, 0), ent(4 * (size_t)T);
-    if (p.solver_type == XPBD_SOLVER_JACOBI && p.jacobi_variant == XPBD_JACOBI_GATHER) {
-        for (int sidx = 0; sidx < T; sidx++) {
-            const int4 e = hidx[sidx];
-            off[e.x + 1]++; off[e.y + 1]++; off[e.z + 1]++; off[e.w + 1]++;
-        }
-        for (int i = 0; i < V; i++) off[i + 1] += off[i];
-        std::vector<int> fill(off.begin(), off.end() - 1);
-        for (int sidx = 0; sidx < T; sidx++) {
-            const int4 e = hidx[sidx];
-            const int vs[4] = {e.x, e.y, e.z, e.w};
-            for (int k = 0; k < 4; k++) ent[fill[vs[k]]++] = 4 * sidx + k;
-        }
-    }
-
     // device allocation + upload
     XPBD_CU(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     {
@@ -1333,11 +1387,8 @@ int build(xpbd_ctx* c, const xpbd_mesh_desc* ms, int n_inst) {
         XPBD_CU(c, cudaMemcpy(c->patch_verts.p, pverts.data(), sizeof(int4) * pverts.size(), cudaMemcpyHostToDevice));
     }
     if (p.solver_type == XPBD_SOLVER_JACOBI && p.jacobi_variant == XPBD_JACOBI_GATHER) {
-        XPBD_CU(c, c->dxt.alloc(3 * (size_t)T));
-        XPBD_CU(c, c->csr_off.alloc(V + 1));
-        XPBD_CU(c, c->csr_ent.alloc(4 * (size_t)T));
-        XPBD_CU(c, cudaMemcpy(c->csr_off.p, off.data(), sizeof(int) * (V + 1), cudaMemcpyHostToDevice));
-        XPBD_CU(c, cudaMemcpy(c->csr_ent.p, ent.data(), sizeof(int) * 4 * (size_t)T, cudaMemcpyHostToDevice));
+        int st = build_jacobi_blocks(c, hidx);
+        if (st) return st;
     }
     XPBD_CU(c, cudaMemcpy(c->tet_idx.p, hidx.data(), sizeof(int4) * T, cudaMemcpyHostToDevice));
     XPBD_CU(c, cudaMemcpy(c->q0.p, h0.data(), sizeof(float4) * T, cudaMemcpyHostToDevice));
@@ -1353,7 +1404,7 @@ int build(xpbd_ctx* c, const xpbd_mesh_desc* ms, int n_inst) {
     XPBD_CU(c, cudaMemset(c->dx.p, 0, sizeof(float4) * V));
     XPBD_CU(c, cudaMemset(c->vel.p, 0, sizeof(float4) * V));
     XPBD_CU(c, cudaMemset(c->flags.p, 0, sizeof(Flags)));
-    c->res_stride = residual_blocks(T, c->block) + 1;
+    c->res_stride = std::max(residual_blocks(T, c->block), c->jb.nblocks) + 1;
     int st = stage_positions_to_device(c, X, nullptr);
     if (st) return st;
     XPBD_CU(c, cudaMemcpy(c->prev.p, c->x.p, sizeof(float4) * V, cudaMemcpyDeviceToDevice));

@@ -270,7 +270,10 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     const bool fuse_final = !track && !local && !solve_only;
     const bool final_on_chip = fuse_predict && fuse_final;
     if (jacobi) {
-        const bool gather = p.jacobi_variant == XPBD_JACOBI_GATHER;
+        // by blocks of tets with partial sums (JACOBI_GATHER), or with vector
+        // atomics into dx
+        const bool blocks = c->jb.nblocks > 0;
+        const bool extra = have_static || c->self_on || c->nbodies || !c->att_v.empty();
         if (track && !every_iter && !warm) exact_residual_row(c, 0, false);
         for (int it = 0; it < iters; it++) {
             // a warm start keeps its multipliers: no iteration treats lambda as 0
@@ -278,62 +281,40 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
             const bool first_contact = it == 0;
             const ResidualSink rs = every_iter && !(warm && it == 0) ? sink(c, it, 0) : no_sink();
             const bool last = it == iters - 1;
-            if (gather) {
-                {
-                    Scope sc(c, K_PROJECT_JACOBI);
-                    launch_project_jacobi_gather_write(c->L(), c->block, c->tets(), c->T, c->x.p, c->dxt.p, first,
-                                                       separate, rs, c->flags.p);
-                }
-                if (have_static) {
-                    Scope sc(c, K_CONTACT);
-                    launch_contacts_jacobi(c->L(), ca, c->x.p, c->dx.p, first_contact);
-                }
-                if (c->self_on) {
-                    Scope sc(c, K_CONTACT);
-                    launch_self_contacts(c->L(), c->selfs(), c->faces.p, c->x.p, c->dx.p, true, first_contact,
-                                         self_alpha_tilde(c), c->flags.p);
-                }
-                if (c->nbodies) {
-                    Scope sc(c, K_CONTACT);
-                    launch_rigid_contacts(c->L(), ca, c->rc_list.p, c->rc_count.p, c->sphere_tab.p, c->face_inst.p,
-                                          c->rb.p, c->nbodies, c->x.p, c->dx.p, true, first_contact, c->flags.p);
-                }
-                if (!c->att_v.empty()) {
-                    Scope sc(c, K_CONTACT);
-                    launch_attach_jacobi(c->L(), c->d_att_v.p, c->d_att_target.p, c->d_att_lam.p,
-                                         (int)c->att_v.size(), c->x.p, c->dx.p, first_contact);
-                }
-                Scope sc(c, K_GATHER);
-                launch_gather_apply(c->L(), c->x.p, c->dxt.p, c->csr_off.p, c->csr_ent.p, c->dx.p, c->V, c->prev.p,
-                                    c->vel.p, last && fuse_final, dt, write_vel);
-            } else {
-                {
-                    Scope sc(c, K_PROJECT_JACOBI);
+            {
+                Scope sc(c, K_PROJECT_JACOBI);
+                if (blocks)
+                    launch_jacobi_blocks(c->L(), c->tets(), c->jb, c->x.p, c->jb_part.p, first, it > 0, separate, rs,
+                                         c->flags.p);
+                else
                     launch_project_jacobi(c->L(), c->block, c->tets(), c->T, c->x.p, c->dx.p, first, separate, rs,
                                           c->flags.p);
-                }
-                if (have_static) {
-                    Scope sc(c, K_CONTACT);
-                    launch_contacts_jacobi(c->L(), ca, c->x.p, c->dx.p, first_contact);
-                }
-                if (c->self_on) {
-                    Scope sc(c, K_CONTACT);
-                    launch_self_contacts(c->L(), c->selfs(), c->faces.p, c->x.p, c->dx.p, true, first_contact,
-                                         self_alpha_tilde(c), c->flags.p);
-                }
-                if (c->nbodies) {
-                    Scope sc(c, K_CONTACT);
-                    launch_rigid_contacts(c->L(), ca, c->rc_list.p, c->rc_count.p, c->sphere_tab.p, c->face_inst.p,
-                                          c->rb.p, c->nbodies, c->x.p, c->dx.p, true, first_contact, c->flags.p);
-                }
-                if (!c->att_v.empty()) {
-                    Scope sc(c, K_CONTACT);
-                    launch_attach_jacobi(c->L(), c->d_att_v.p, c->d_att_target.p, c->d_att_lam.p,
-                                         (int)c->att_v.size(), c->x.p, c->dx.p, first_contact);
-                }
-                Scope sc(c, K_APPLY);
-                launch_apply(c->L(), c->x.p, c->dx.p, c->V, c->prev.p, c->vel.p, last && fuse_final, dt, write_vel);
             }
+            if (have_static) {
+                Scope sc(c, K_CONTACT);
+                launch_contacts_jacobi(c->L(), ca, c->x.p, c->dx.p, first_contact);
+            }
+            if (c->self_on) {
+                Scope sc(c, K_CONTACT);
+                launch_self_contacts(c->L(), c->selfs(), c->faces.p, c->x.p, c->dx.p, true, first_contact,
+                                     self_alpha_tilde(c), c->flags.p);
+            }
+            if (c->nbodies) {
+                Scope sc(c, K_CONTACT);
+                launch_rigid_contacts(c->L(), ca, c->rc_list.p, c->rc_count.p, c->sphere_tab.p, c->face_inst.p,
+                                      c->rb.p, c->nbodies, c->x.p, c->dx.p, true, first_contact, c->flags.p);
+            }
+            if (!c->att_v.empty()) {
+                Scope sc(c, K_CONTACT);
+                launch_attach_jacobi(c->L(), c->d_att_v.p, c->d_att_target.p, c->d_att_lam.p, (int)c->att_v.size(),
+                                     c->x.p, c->dx.p, first_contact);
+            }
+            Scope sc(c, blocks ? K_GATHER : K_APPLY);
+            if (blocks)
+                launch_jacobi_gather(c->L(), c->x.p, c->jb_part.p, c->jb, c->dx.p, extra, c->V, c->prev.p, c->vel.p,
+                                     last && fuse_final, dt, write_vel);
+            else
+                launch_apply(c->L(), c->x.p, c->dx.p, c->V, c->prev.p, c->vel.p, last && fuse_final, dt, write_vel);
         }
     } else if (cluster) {
         if (track && !warm) exact_residual_row(c, 0, false);

@@ -69,12 +69,16 @@ struct xpbd_ctx {
     std::vector<float> alpha_t_d, alpha_t_h;  // per slot, for energy
 
     // device state
-    DevBuf<float4> x, prev, vel, dx, dxt;
+    DevBuf<float4> x, prev, vel, dx;
+    // Jacobi by blocks: the tables in one buffer, the partial sums
+    DevBuf<int4> jb_tab;
+    DevBuf<float4> jb_part;
+    xg::JacobiBlocks jb{};
     DevBuf<int4> tet_idx;
     DevBuf<float4> m0, m1, m2;  // projection records (M = Q Q^T, det Q, compliances)
     DevBuf<float4> q0, q1, q2;  // Q, for the network features
     DevBuf<float2> lam;
-    DevBuf<int> perm, csr_off, csr_ent;
+    DevBuf<int> perm;
     DevBuf<int4> faces;
     DevBuf<int> face_list;
     DevBuf<int4> patch_meta, patch_verts;

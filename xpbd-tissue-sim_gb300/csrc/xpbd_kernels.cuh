@@ -63,6 +63,20 @@ struct ContactArrays {
     int S;
 };
 
+// Jacobi: blocks of consecutive slots with their vertices (k_jacobi_blocks)
+constexpr int kJacobiTets = 160;   // tets of a block, one thread each (32 hexes of five)
+constexpr int kJacobiVerts = 256;  // its vertices at most
+struct JacobiBlocks {
+    const int4* block;           // [nblocks] first slot, tets, first vertex entry, vertices
+    const int* vert;             // [entries] the blocks' vertices
+    const uchar4* corner;        // [T] a tet's vertices as indices into its block's
+    const unsigned* range;       // [entries] a vertex's part of its block's corner list: first << 16 | count
+    const unsigned short* list;  // [4 T] the blocks' corner lists (4 x first slot on): 4 x tet in the block + corner
+    const int* voff;             // [V + 1] CSR vertex -> entries
+    const int* vent;             // [entries]
+    int nblocks;
+};
+
 // Gauss-Seidel patches: up to kMaxPatchTets consecutive tets on at most
 // kMaxPatchVerts vertices, one thread each.
 constexpr int kMaxPatchTets = 5;
@@ -318,10 +332,12 @@ void launch_kinematic(const Launch& s, float4* x, const int* idx, const float4* 
                       float oz);
 void launch_project_jacobi(const Launch& s, int block, const TetArrays& t, int T, const float4* x, float4* dx,
                            bool first, bool separate, ResidualSink res, Flags* flags);
-void launch_project_jacobi_gather_write(const Launch& s, int block, const TetArrays& t, int T, const float4* x,
-                                        float4* dxt, bool first, bool separate, ResidualSink res, Flags* flags);
-void launch_gather_apply(const Launch& s, float4* x, const float4* dxt, const int* csr_off, const int* csr_ent,
-                         float4* dx, int V, float4* prev, float4* vel, bool final_step, float dt, bool write_vel);
+// lam_early: the launch before this one on the stream does not write the multipliers
+void launch_jacobi_blocks(const Launch& s, const TetArrays& t, const JacobiBlocks& jb, const float4* x, float4* part,
+                          bool first, bool lam_early, bool separate, ResidualSink res, Flags* flags);
+// extra: dx holds updates too (contacts, attachments)
+void launch_jacobi_gather(const Launch& s, float4* x, const float4* part, const JacobiBlocks& jb, float4* dx,
+                          bool extra, int V, float4* prev, float4* vel, bool final_step, float dt, bool write_vel);
 void launch_apply(const Launch& s, float4* x, float4* dx, int V, float4* prev, float4* vel, bool final_step,
                   float dt, bool write_vel);
 void launch_project_patches(const Launch& s, const TetArrays& t, const PatchArrays& pa, int pbegin, int pend,
