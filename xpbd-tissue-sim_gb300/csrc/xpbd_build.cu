@@ -131,7 +131,7 @@ void release(xpbd_ctx* c) {
     c->mlp_p.release(); c->mlp_m.release(); c->mlp_v.release(); c->mlp_g.release(); c->mlp_w4f.release();
     c->mlp_tiles.release(); c->mat.release(); c->feat.release(); c->pred.release(); c->target.release();
     c->x_pred.release(); c->warm_stats.release(); c->warm_rows.release(); c->mse.release();
-    c->cache_z.release(); c->cache_out.release(); c->cache_a.release();
+    c->cache_z.release(); c->cache_out.release();
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_rows) cudaFreeHost(c->h_rows);
     c->h_stage = nullptr;

@@ -221,7 +221,6 @@ struct xpbd_ctx {
     DevBuf<double> warm_rows, mse;     // 2 residual sums; loss accumulator
     int cache_rows = 0;                // training cache capacity (rows)
     DevBuf<float> cache_z, cache_out;
-    DevBuf<__nv_bfloat16> cache_a;
 
     xg::MlpNet net() {
         __nv_bfloat16* b = mlp_tiles.p;

@@ -310,8 +310,7 @@ struct MlpNet {
 };
 
 struct MlpCache {
-    float* z[3];            // pre-activations of the hidden layers, [n][64]
-    __nv_bfloat16* a[3];    // their BF16 activations, [n][64]
+    float* z[3];            // pre-activations of the hidden layers, [ceil(n / 128)][64][128]
 };
 
 cudaError_t mlp_prepare_kernels();

@@ -165,6 +165,13 @@ constexpr int kW4Bytes = kOutPad * kHid * 2;   // 16 x 64
 constexpr int kA0Bytes = kRows * kIn * 2;      // 128 x 16
 constexpr int kABytes = kRows * kHid * 2;      // 128 x 64
 
+// The training cache: the hidden layers' pre-activations by tile, column, row,
+// so that the 32 rows of a warp lie together. (The activations follow from them
+// by the forward pass's own arithmetic and are not kept.)
+__device__ __forceinline__ size_t zcache(int tile, int col, int row) {
+    return ((size_t)tile * kHid + col) * kRows + row;
+}
+
 // ---- forward: persistent CTAs, one 128-tet tile at a time ----
 // Smem: W1 | W2 | W3 | W4 | A0 | A  (+ biases, barrier, tmem address). The
 // weights and biases are staged once per CTA; each tile's input rows are
@@ -266,17 +273,10 @@ __global__ void __launch_bounds__(kFwdThreads) k_mlp_forward(const __nv_bfloat16
                     for (int i = 0; i < 16; i++) {
                         const float z = v[i] + bl[c + i];
                         a[i] = silu_f(z);
-                        if (TRAIN && live) cache.z[layer][(size_t)row * kHid + c + i] = z;
+                        if (TRAIN) cache.z[layer][zcache(tile, c + i, t)] = z;
                     }
                     st_row8(A, t, c, kHid, a);
                     st_row8(A, t, c + 8, kHid, a + 8);
-                    if (TRAIN && live) {
-                        // the BF16 activation the next layer consumes
-                        *reinterpret_cast<uint4*>(cache.a[layer] + (size_t)row * kHid + c) =
-                            *reinterpret_cast<const uint4*>(A + kmaj_off(t, c, kHid));
-                        *reinterpret_cast<uint4*>(cache.a[layer] + (size_t)row * kHid + c + 8) =
-                            *reinterpret_cast<const uint4*>(A + kmaj_off(t, c + 8, kHid));
-                    }
                 }
                 async_smem_fence();
                 tc_before();
@@ -306,105 +306,159 @@ __global__ void __launch_bounds__(kFwdThreads) k_mlp_forward(const __nv_bfloat16
     if (warp == 0) tmem_dealloc(tmem, 64);
 }
 
-// ---- backward: `tiles` consecutive 128-row tiles per CTA ----
+// ---- backward: persistent CTAs, one 128-row tile at a time ----
 // Smem: W3t | W2t | Td (128x64) | TdT (128x128) | TaT (64x128)
 constexpr int kTdTBytes = kRows * kRows * 2;
 constexpr int kTaTBytes = kHid * kRows * 2;
 constexpr int kBwdSmem = 2 * kW2Bytes + kABytes + kTdTBytes + kTaTBytes;
+constexpr int kBwdThreads = 2 * kRows;
+constexpr int kCols = kHid / 2;  // hidden columns of a thread
 
-__global__ void __launch_bounds__(kRows) k_mlp_backward(const __nv_bfloat16* __restrict__ X, const float* __restrict__ Y,
-                                                        int n, int tiles, float inv_batch, MlpNet net, MlpCache cache,
-                                                        const float* __restrict__ out, float* __restrict__ grad,
-                                                        unsigned long long* __restrict__ err) {
+// v[i] of the warp's lanes added up for every i < 32,
+// by halving: 31 shuffles instead of 160. Lane l returns column l's sum in v[0].
+__device__ __forceinline__ void warp_columns(float (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16, n = 32; o > 0; o >>= 1, n >>= 1) {
+        const bool hi = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n / 2; i++) {
+            const float send = hi ? v[i] : v[i + n / 2], keep = hi ? v[i + n / 2] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+}
+
+// Bound by its epilogues, not by the products (6 MMA chains of 128x64x128 or
+// less a tile): what counts is the z cache's access and the column sums.
+// Each CTA keeps dW3, dW2, dW1 in tensor memory and the bias and W4 sums in
+// registers over all its tiles and adds them to grad once (vector reductions).
+// 65,536 rows: 283 us with a CTA a tile, row-major caches and a full warp sum
+// for each of the 320 columns of a tile; 40 us now (forward with its cache 86 -> 20).
+__global__ void __launch_bounds__(kBwdThreads, 2) k_mlp_backward(const __nv_bfloat16* __restrict__ X,
+                                                              const float* __restrict__ Y, int n, float inv_batch,
+                                                              MlpNet net, MlpCache cache,
+                                                              const float* __restrict__ out, float* __restrict__ grad,
+                                                              unsigned long long* __restrict__ err) {
     extern __shared__ __align__(128) char smem[];
     __shared__ __align__(8) unsigned long long bar;
     __shared__ unsigned s_tmem;
-    __shared__ float s_g4[kOutPad * kHid];  // dW4 (2 x 64 used)
-    __shared__ float s_gb[3 * kHid + 2];    // db1, db2, db3, db4
+    __shared__ float s_w4[2 * kHid];
+    __shared__ float s_sum[5 * kHid + 2];  // db1, db2, db3, dW4 (2 x 64), db4
     char* W3t = smem;
     char* W2t = W3t + kW2Bytes;
     char* Td = W2t + kW2Bytes;
     char* TdT = Td + kABytes;
     char* TaT = TdT + kTdTBytes;
-    const int t = threadIdx.x, warp = t >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t = (warp & 3) * 32 + lane;  // row within the tile
+    const int c0 = kCols * (warp >> 2);    // this thread's hidden columns c0 .. c0 + 31
+    const int ntiles = (n + kRows - 1) / kRows;
     copy_smem(W3t, (const char*)net.w3t, kW2Bytes);
     copy_smem(W2t, (const char*)net.w2t, kW2Bytes);
     zero_smem(TdT, kTdTBytes);  // rows 64..127 (the M padding) stay zero
-    for (int i = t; i < kOutPad * kHid; i += kRows) s_g4[i] = 0.f;
-    for (int i = t; i < 3 * kHid + 2; i += kRows) s_gb[i] = 0.f;
-    if (t == 0) bar_init(&bar);
+    for (int i = threadIdx.x; i < 5 * kHid + 2; i += kBwdThreads) s_sum[i] = 0.f;
+    for (int i = threadIdx.x; i < 2 * kHid; i += kBwdThreads) s_w4[i] = __ldg(net.w4f + i);
+    if (threadIdx.x == 0) bar_init(&bar);
     if (warp == 0) tmem_alloc(&s_tmem, 256);
     async_smem_fence();
     tc_before();
     __syncthreads();
     tc_after();
     const unsigned tmem = s_tmem;
-    const unsigned my_lane = tmem + ((unsigned)(32 * warp) << 16);
+    const unsigned my_lane = tmem + ((unsigned)(32 * (warp & 3)) << 16);
     // columns: [0,64) dA scratch, [64,128) dW3, [128,192) dW2, [192,208) dW1
     unsigned phase = 0;
     bool ok = true;
-    for (int tile = 0; tile < tiles && ok; tile++) {
-        const int row = (blockIdx.x * tiles + tile) * kRows + t;
+    float gb[3] = {0.f, 0.f, 0.f}, g4[2] = {0.f, 0.f}, gb4[2] = {0.f, 0.f};  // of column c0 + lane
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const int row = tile * kRows + t;
         const bool live = row < n;
-        // output layer (2 wide) on the CUDA cores
+        // output layer (2 wide) on the CUDA cores; rows past the end have d4 = 0,
+        // so every gradient of theirs is 0
         float d4[2] = {0.f, 0.f};
         if (live) {
-            d4[0] = 2.f * (out[2 * (size_t)row] - Y[2 * (size_t)row]) * inv_batch;
-            d4[1] = 2.f * (out[2 * (size_t)row + 1] - Y[2 * (size_t)row + 1]) * inv_batch;
+            const float2 o = *reinterpret_cast<const float2*>(out + 2 * (size_t)row);
+            const float2 y = *reinterpret_cast<const float2*>(Y + 2 * (size_t)row);
+            d4[0] = 2.f * (o.x - y.x) * inv_batch;
+            d4[1] = 2.f * (o.y - y.y) * inv_batch;
         }
-        warp_add(&s_gb[3 * kHid], d4[0]);
-        warp_add(&s_gb[3 * kHid + 1], d4[1]);
-        float d[kHid];
+        if (c0 == 0) {
+            gb4[0] += d4[0];
+            gb4[1] += d4[1];
+        }
+        float d[kCols];
+        {
+            float z[kCols];
 #pragma unroll
-        for (int i = 0; i < kHid; i++) {
-            const float a3 = live ? __bfloat162float(cache.a[2][(size_t)row * kHid + i]) : 0.f;
-            warp_add(&s_g4[i], d4[0] * a3);
-            warp_add(&s_g4[kHid + i], d4[1] * a3);
-            const float da3 = d4[0] * __ldg(net.w4f + i) + d4[1] * __ldg(net.w4f + kHid + i);
-            d[i] = live ? da3 * dsilu_f(cache.z[2][(size_t)row * kHid + i]) : 0.f;
+            for (int i = 0; i < kCols; i++) z[i] = cache.z[2][zcache(tile, c0 + i, t)];
+#pragma unroll
+            for (int i = 0; i < kCols; i++) {
+                if (!live) z[i] = 0.f;
+                const float da3 = d4[0] * s_w4[c0 + i] + d4[1] * s_w4[kHid + c0 + i];
+                d[i] = da3 * dsilu_f(z[i]);
+                z[i] = __bfloat162float(__float2bfloat16_rn(silu_f(z[i])));  // the activation W4 saw
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                float w[kCols];
+#pragma unroll
+                for (int i = 0; i < kCols; i++) w[i] = d4[k] * z[i];
+                warp_columns(w);
+                g4[k] += w[0];
+            }
         }
         // layers 3, 2, 1: dA = D W (tensor cores), dW += D^T A (tensor cores)
-        for (int layer = 2; layer >= 0 && ok; layer--) {
 #pragma unroll
-            for (int i = 0; i < kHid; i++) warp_add(&s_gb[layer * kHid + i], d[i]);
-#pragma unroll
-            for (int c = 0; c < kHid; c += 8) st_row8(Td, t, c, kHid, d + c);
-#pragma unroll
-            for (int i = 0; i < kHid; i++) st_one(TdT, i, t, kRows, d[i]);
-            const int in_w = layer == 0 ? kIn : kHid;
+        for (int layer = 2; layer >= 0; layer--) {
+            float ds[kCols];  // the SiLU derivative of the layer below
             if (layer > 0) {
-                for (int i = 0; i < kHid; i++) {
-                    const float a = live ? __bfloat162float(cache.a[layer - 1][(size_t)row * kHid + i]) : 0.f;
-                    st_one(TaT, i, t, kRows, a);
+#pragma unroll
+                for (int i = 0; i < kCols; i++) {
+                    float z = cache.z[layer - 1][zcache(tile, c0 + i, t)];
+                    if (!live) z = 0.f;
+                    st_one(TaT, c0 + i, t, kRows, silu_f(z));
+                    ds[i] = dsilu_f(z);
                 }
-            } else {
-                for (int i = 0; i < kIn; i++) {
-                    const float a = live ? __bfloat162float(X[(size_t)row * kIn + i]) : 0.f;
-                    st_one(TaT, i, t, kRows, a);
+            } else if (c0 == 0) {
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    uint4 r = make_uint4(0, 0, 0, 0);
+                    if (live) r = __ldg(reinterpret_cast<const uint4*>(X + (size_t)row * kIn + 8 * q));
+                    const unsigned u[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        *reinterpret_cast<unsigned short*>(TaT + kmaj_off(8 * q + k, t, kRows)) =
+                            (unsigned short)(u[k >> 1] >> (16 * (k & 1)));
                 }
             }
+#pragma unroll
+            for (int c = 0; c < kCols; c += 8) st_row8(Td, t, c0 + c, kHid, d + c);
+#pragma unroll
+            for (int i = 0; i < kCols; i++) st_one(TdT, c0 + i, t, kRows, d[i]);
             async_smem_fence();
             tc_before();
             __syncthreads();
             tc_after();
-            if (t == 0) {
+            if (threadIdx.x == 0) {
                 const unsigned col = layer == 2 ? 64u : (layer == 1 ? 128u : 192u);
-                mma_tile(tmem + col, TdT, TaT, kRows, in_w, tile > 0);
+                mma_tile(tmem + col, TdT, TaT, kRows, layer == 0 ? kIn : kHid, tile != (int)blockIdx.x);
                 if (layer > 0) mma_tile(tmem, Td, layer == 2 ? W3t : W2t, kHid, kHid, false);
                 umma_commit(&bar);
             }
+            warp_columns(d);  // the bias gradient, while the products run
+            gb[layer] += d[0];
             ok = __syncthreads_and(bar_wait(&bar, phase)) != 0;
             phase ^= 1u;
             tc_after();
             if (!ok) break;
             if (layer > 0) {
 #pragma unroll
-                for (int c = 0; c < kHid; c += 16) {
+                for (int c = 0; c < kCols; c += 16) {
                     float v[16];
-                    tmem_ld16(my_lane + c, v);
+                    tmem_ld16(my_lane + c0 + c, v);
 #pragma unroll
-                    for (int i = 0; i < 16; i++)
-                        d[c + i] = live ? v[i] * dsilu_f(cache.z[layer - 1][(size_t)row * kHid + c + i]) : 0.f;
+                    for (int i = 0; i < 16; i++) d[c + i] = v[i] * ds[c + i];
                 }
             }
             tc_before();
@@ -412,31 +466,46 @@ __global__ void __launch_bounds__(kRows) k_mlp_backward(const __nv_bfloat16* __r
             tc_after();
         }
     }
-    if (ok) {
+    if (ok && (int)blockIdx.x < ntiles) {
         // weight gradients out of tensor memory: rows j < 64 live in lanes 0..63
-        if (warp < 2) {
+        if ((warp & 3) < 2) {
             const int j = t;
-            for (int c = 0; c < kHid; c += 16) {
-                float v[16];
-                tmem_ld16(my_lane + 64 + c, v);
-                for (int i = 0; i < 16; i++) atomicAdd(grad + kOffW3 + j * kHid + c + i, v[i]);
-                tmem_ld16(my_lane + 128 + c, v);
-                for (int i = 0; i < 16; i++) atomicAdd(grad + kOffW2 + j * kHid + c + i, v[i]);
-            }
+            auto add16 = [&](float* g, const float* v) {
+#pragma unroll
+                for (int i = 0; i < 16; i += 4)
+                    atomicAdd(reinterpret_cast<float4*>(g + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+            };
             float v[16];
-            tmem_ld16(my_lane + 192, v);
-            for (int i = 0; i < kIn; i++) atomicAdd(grad + kOffW1 + j * kIn + i, v[i]);
+            for (int c = c0; c < c0 + kCols; c += 16) {
+                tmem_ld16(my_lane + 64 + c, v);
+                add16(grad + kOffW3 + j * kHid + c, v);
+                tmem_ld16(my_lane + 128 + c, v);
+                add16(grad + kOffW2 + j * kHid + c, v);
+            }
+            if (c0 == 0) {
+                tmem_ld16(my_lane + 192, v);
+                add16(grad + kOffW1 + j * kIn, v);
+            }
+        }
+        // the warps' column sums, then one addition a block
+#pragma unroll
+        for (int k = 0; k < 3; k++) atomicAdd(&s_sum[k * kHid + c0 + lane], gb[k]);
+#pragma unroll
+        for (int k = 0; k < 2; k++) atomicAdd(&s_sum[(3 + k) * kHid + c0 + lane], g4[k]);
+        if (c0 == 0) {
+            warp_add(&s_sum[5 * kHid], gb4[0]);
+            warp_add(&s_sum[5 * kHid + 1], gb4[1]);
         }
         __syncthreads();
-        for (int i = t; i < 2 * kHid; i += kRows) atomicAdd(grad + kOffW4 + i, s_g4[i]);
-        for (int i = t; i < kHid; i += kRows) {
-            atomicAdd(grad + kOffB1 + i, s_gb[i]);
-            atomicAdd(grad + kOffB2 + i, s_gb[kHid + i]);
-            atomicAdd(grad + kOffB3 + i, s_gb[2 * kHid + i]);
+        for (int i = threadIdx.x; i < kHid; i += kBwdThreads) {
+            atomicAdd(grad + kOffB1 + i, s_sum[i]);
+            atomicAdd(grad + kOffB2 + i, s_sum[kHid + i]);
+            atomicAdd(grad + kOffB3 + i, s_sum[2 * kHid + i]);
         }
-        if (t < 2) atomicAdd(grad + kOffB4 + t, s_gb[3 * kHid + t]);
-    } else {
-        if (t == 0) atomicAdd(err, 1ull);
+        for (int i = threadIdx.x; i < 2 * kHid; i += kBwdThreads) atomicAdd(grad + kOffW4 + i, s_sum[3 * kHid + i]);
+        if (threadIdx.x < 2) atomicAdd(grad + kOffB4 + threadIdx.x, s_sum[5 * kHid + threadIdx.x]);
+    } else if (!ok) {
+        if (threadIdx.x == 0) atomicAdd(err, 1ull);
         bar_wait(&bar, 0);
         bar_wait(&bar, 1);
     }
@@ -501,6 +570,17 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ Y
 
 inline int nb(long long n, int b) { return (int)((n + b - 1) / b); }
 
+int sm_count() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+            n = 148;
+        return n;
+    }();
+    return sms;
+}
+
 }  // namespace
 
 int mlp_forward_smem() { return kFwdSmem; }
@@ -525,14 +605,7 @@ void launch_mlp_forward(cudaStream_t s, const __nv_bfloat16* X, int n, const Mlp
     // persistent: 5 CTAs per SM (shared memory's limit; 64 tensor-memory columns each),
     // weights staged once each; co-resident CTAs overlap one another's MMA waits with
     // their epilogues (0.104 ms with 4 per SM, 0.099 with 5, 1.31M rows)
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    const int grid = std::min(nb(n, kRows), 5 * sms);
+    const int grid = std::min(nb(n, kRows), 5 * sm_count());
     if (cache)
         k_mlp_forward<true><<<grid, kFwdThreads, kFwdSmem, s>>>(X, n, net, out, *cache, err);
     else
@@ -542,10 +615,9 @@ void launch_mlp_forward(cudaStream_t s, const __nv_bfloat16* X, int n, const Mlp
 void launch_mlp_backward(cudaStream_t s, const __nv_bfloat16* X, const float* Y, int n, const MlpNet& net,
                          const MlpCache& cache, const float* out, float* grad, unsigned long long* err) {
     if (n <= 0) return;
-    const int tiles_total = nb(n, kRows);
-    const int tiles = tiles_total >= 8 * 148 ? 8 : 1;
-    k_mlp_backward<<<nb(tiles_total, tiles), kRows, kBwdSmem, s>>>(X, Y, n, tiles, 1.f / (float)n, net, cache, out,
-                                                                  grad, err);
+    // two CTAs an SM (shared memory and tensor memory), each with several tiles
+    const int grid = std::min(nb(n, kRows), 2 * sm_count());
+    k_mlp_backward<<<grid, kBwdThreads, kBwdSmem, s>>>(X, Y, n, 1.f / (float)n, net, cache, out, grad, err);
 }
 
 void launch_mse(cudaStream_t s, const float* out, const float* Y, int n, double* acc) {

@@ -88,10 +88,9 @@ int ensure_cache(xpbd_ctx* c, int rows) {
     if (c->cache_rows >= rows) return XPBD_OK;
     XPBD_CU(c, cudaStreamSynchronize(c->stream));
     c->cache_z.release();
-    c->cache_a.release();
     c->cache_out.release();
+    rows = (rows + 127) / 128 * 128;  // the cache holds whole tiles
     XPBD_CU(c, c->cache_z.alloc(3 * (size_t)kMlpHid * rows));
-    XPBD_CU(c, c->cache_a.alloc(3 * (size_t)kMlpHid * rows));
     XPBD_CU(c, c->cache_out.alloc(2 * (size_t)rows));
     c->cache_rows = rows;
     return XPBD_OK;
@@ -99,8 +98,7 @@ int ensure_cache(xpbd_ctx* c, int rows) {
 
 MlpCache cache_of(xpbd_ctx* c) {
     const size_t r = (size_t)c->cache_rows * kMlpHid;
-    return MlpCache{{c->cache_z.p, c->cache_z.p + r, c->cache_z.p + 2 * r},
-                    {c->cache_a.p, c->cache_a.p + r, c->cache_a.p + 2 * r}};
+    return MlpCache{{c->cache_z.p, c->cache_z.p + r, c->cache_z.p + 2 * r}};
 }
 
 // one forward (training) + loss + backward on device rows [X, Y) of n rows;
