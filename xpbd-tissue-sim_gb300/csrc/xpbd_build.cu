@@ -134,6 +134,9 @@ void release(xpbd_ctx* c) {
     c->cache_z.release(); c->cache_out.release();
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_rows) cudaFreeHost(c->h_rows);
+    if (c->h_mlp) cudaFreeHost(c->h_mlp);
+    c->h_mlp = nullptr;
+    c->mlp_rows.release();
     c->h_stage = nullptr;
     c->h_rows = nullptr;
     if (c->stream) cudaStreamDestroy(c->stream);

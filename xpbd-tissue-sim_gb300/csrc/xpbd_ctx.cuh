@@ -32,6 +32,13 @@ struct DevBuf {
     }
 };
 
+// what a loss / gradient call copies back (pinned)
+struct MlpResults {
+    Flags flags;
+    double loss;
+    float grad[kMlpParams];
+};
+
 struct Prof {
     bool on = false;
     std::vector<cudaEvent_t> pool;
@@ -43,6 +50,7 @@ struct Prof {
 
 using xg::DevBuf;
 using xg::Flags;
+using xg::MlpResults;
 using xg::Launch;
 using xg::PatchArrays;
 using xg::Prof;
@@ -219,6 +227,8 @@ struct xpbd_ctx {
     DevBuf<float4> x_pred;             // V: predicted positions (fallback restore)
     DevBuf<unsigned long long> warm_stats;  // kept, rejected warm starts
     DevBuf<double> warm_rows, mse;     // 2 residual sums; loss accumulator
+    DevBuf<uint4> mlp_rows;            // rows of the calls on host arrays
+    MlpResults* h_mlp = nullptr;
     int cache_rows = 0;                // training cache capacity (rows)
     DevBuf<float> cache_z, cache_out;
 

@@ -61,7 +61,41 @@ __global__ void __launch_bounds__(kHostIoThreads) k_xyz_to_host(H* __restrict__ 
     }
 }
 
+// The network's rows (16 floats) as BF16 and their targets (2 floats), read from
+// host arrays the device addresses: eight values a thread, in 16-byte pieces
+// where the arrays are aligned to them. (Rounding on one host core, a fresh
+// device buffer and a pageable copy took 0.5 of the 0.64 ms of a loss and
+// gradient call on 65,536 rows.)
+__global__ void __launch_bounds__(256) k_rows_from_host(__nv_bfloat16* __restrict__ X, const float* __restrict__ hX,
+                                                        float* __restrict__ Y, const float* __restrict__ hY,
+                                                        long long n) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 2 * n) {
+        float v[8];
+        const float* p = hX + 8 * i;
+        if (((uintptr_t)hX & 15) == 0) {
+            const float4 a = __ldcv(reinterpret_cast<const float4*>(p)), b = __ldcv(reinterpret_cast<const float4*>(p) + 1);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        } else {
+            for (int k = 0; k < 8; k++) v[k] = __ldcv(p + k);
+        }
+        __nv_bfloat162 h[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) h[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+        reinterpret_cast<uint4*>(X)[i] = *reinterpret_cast<const uint4*>(h);
+        if (Y && i < n) {
+            Y[2 * i] = __ldcv(hY + 2 * i);
+            Y[2 * i + 1] = __ldcv(hY + 2 * i + 1);
+        }
+    }
+}
+
 }  // namespace
+
+void launch_rows_from_host(cudaStream_t s, __nv_bfloat16* X, const float* hX, float* Y, const float* hY, long long n) {
+    if (n > 0) k_rows_from_host<<<nblk(2 * n, 256), 256, 0, s>>>(X, hX, Y, hY, n);
+}
 
 void launch_xyz_from_host(cudaStream_t s, float4* x, const double* h, int V, bool keep_w) {
     if (V > 0) k_xyz_from_host<double><<<nblk(V, kHostIoThreads), kHostIoThreads, 0, s>>>(x, h, V, keep_w);

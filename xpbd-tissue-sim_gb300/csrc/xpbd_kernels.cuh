@@ -427,6 +427,8 @@ void launch_self_contacts(const Launch& s, const SelfArrays& a, const int4* face
 // (keep_w: the float4's w is left as it is; else 0)
 void launch_xyz_from_host(cudaStream_t s, float4* x, const double* h, int V, bool keep_w);
 void launch_xyz_from_host(cudaStream_t s, float4* x, const float* h, int V, bool keep_w);
+// network rows (n x 16) to BF16, and their targets (n x 2; Y may be null)
+void launch_rows_from_host(cudaStream_t s, __nv_bfloat16* X, const float* hX, float* Y, const float* hY, long long n);
 void launch_xyz_to_host(cudaStream_t s, double* h, const float4* x, int V);
 void launch_xyz_to_host(cudaStream_t s, float* h, const float4* x, int V);
 void launch_attach_gs(const Launch& s, const int* vert, const float4* target, float* lam, const int* order, int begin,

@@ -45,6 +45,7 @@ float from_bf16(uint16_t h) {
 int ensure_mlp(xpbd_ctx* c) {
     if (c->mlp_p.p) return XPBD_OK;
     XPBD_CU(c, mlp_prepare_kernels());
+    if (!c->h_mlp) XPBD_CU(c, cudaMallocHost((void**)&c->h_mlp, sizeof(MlpResults)));
     XPBD_CU(c, c->mlp_p.alloc(kMlpParams));
     XPBD_CU(c, c->mlp_m.alloc(kMlpParams));
     XPBD_CU(c, c->mlp_v.alloc(kMlpParams));
@@ -122,24 +123,47 @@ void enqueue_adam(xpbd_ctx* c, float lr) {
     c->launches += 2;
 }
 
-// host FP32 rows (n x 16) -> a fresh device BF16 buffer
-int upload_features(xpbd_ctx* c, const float* X, int64_t n, DevBuf<__nv_bfloat16>& d) {
-    std::vector<uint16_t> h((size_t)n * kMlpIn);
-    for (size_t i = 0; i < h.size(); i++) h[i] = to_bf16(X[i]);
-    XPBD_CU(c, d.alloc(h.size()));
-    XPBD_CU(c, cudaMemcpy(d.p, h.data(), sizeof(uint16_t) * h.size(), cudaMemcpyHostToDevice));
-    return XPBD_OK;
-}
-
-struct Tmp {
-    DevBuf<__nv_bfloat16> X;
-    DevBuf<float> Y, out;
-    ~Tmp() {
-        X.release();
-        Y.release();
-        out.release();
+// Device buffers of a call on host rows. Calls of up to kKeptRows rows (44 bytes
+// each, 46 MB) share the context's, which grow to the largest such call and go
+// with the context; a larger call has its own.
+constexpr int64_t kKeptRows = 1 << 20;
+struct RowBuffers {
+    __nv_bfloat16* X = nullptr;
+    float *Y = nullptr, *out = nullptr;
+    DevBuf<uint4> own;
+    ~RowBuffers() { own.release(); }
+    int get(xpbd_ctx* c, int64_t n) {
+        const size_t need = 2 * (size_t)n + 2 * (((size_t)n + 1) / 2);  // 32 + 8 + 8 bytes a row, in 16s
+        DevBuf<uint4>* d = &own;
+        if (n <= kKeptRows) {
+            d = &c->mlp_rows;
+            if (d->n < need) {
+                XPBD_CU(c, cudaStreamSynchronize(c->stream));
+                d->release();
+            }
+        }
+        if (!d->p) XPBD_CU(c, d->alloc(need));
+        X = reinterpret_cast<__nv_bfloat16*>(d->p);
+        Y = reinterpret_cast<float*>(d->p + 2 * (size_t)n);
+        out = reinterpret_cast<float*>(d->p + 2 * (size_t)n + ((size_t)n + 1) / 2);
+        return XPBD_OK;
     }
 };
+
+// the caller's FP32 rows (n x 16) as BF16, and its targets (n x 2, or null):
+// read by the device itself where it addresses pageable host memory
+int upload_rows(xpbd_ctx* c, const float* X, const float* Y, int64_t n, const RowBuffers& d) {
+    if (c->host_direct) {
+        launch_rows_from_host(c->stream, d.X, X, Y ? d.Y : nullptr, Y, n);
+        return cuda_check(c, cudaGetLastError(), "rows from host");
+    }
+    std::vector<uint16_t> h((size_t)n * kMlpIn);
+    for (size_t i = 0; i < h.size(); i++) h[i] = to_bf16(X[i]);
+    XPBD_CU(c, cudaStreamSynchronize(c->stream));
+    XPBD_CU(c, cudaMemcpy(d.X, h.data(), sizeof(uint16_t) * h.size(), cudaMemcpyHostToDevice));
+    if (Y) XPBD_CU(c, cudaMemcpy(d.Y, Y, sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice));
+    return XPBD_OK;
+}
 
 int check_timeouts(xpbd_ctx* c) {
     Flags f{};
@@ -193,17 +217,18 @@ int xpbd_mlp_get_params(xpbd_ctx* c, float* params, int64_t n) {
 int xpbd_mlp_forward(xpbd_ctx* c, const float* X, int64_t n, float* out) {
     if (!c || !X || !out || n <= 0 || n > (1 << 28)) return XPBD_ERR_INVALID;
     if (!c->mlp_ready) return fail(c, XPBD_ERR_STATE, "network not initialised");
-    Tmp t;
-    int st = upload_features(c, X, n, t.X);
+    RowBuffers t;
+    int st = t.get(c, n);
     if (st) return st;
-    XPBD_CU(c, t.out.alloc(2 * (size_t)n));
-    launch_mlp_forward(c->stream, t.X.p, (int)n, c->net(), t.out.p, nullptr, &c->flags.p->timeouts);
+    st = upload_rows(c, X, nullptr, n, t);
+    if (st) return st;
+    launch_mlp_forward(c->stream, t.X, (int)n, c->net(), t.out, nullptr, &c->flags.p->timeouts);
     c->launches++;
     XPBD_CU(c, cudaGetLastError());
     XPBD_CU(c, cudaStreamSynchronize(c->stream));
     st = check_timeouts(c);
     if (st) return st;
-    XPBD_CU(c, cudaMemcpy(out, t.out.p, sizeof(float) * 2 * (size_t)n, cudaMemcpyDeviceToHost));
+    XPBD_CU(c, cudaMemcpy(out, t.out, sizeof(float) * 2 * (size_t)n, cudaMemcpyDeviceToHost));
     return XPBD_OK;
 }
 
@@ -212,23 +237,25 @@ int xpbd_mlp_loss_grad(xpbd_ctx* c, const float* X, const float* Y, int64_t n, d
     if (!c->mlp_ready) return fail(c, XPBD_ERR_STATE, "network not initialised");
     int st = ensure_cache(c, (int)n);
     if (st) return st;
-    Tmp t;
-    st = upload_features(c, X, n, t.X);
+    RowBuffers t;
+    st = t.get(c, n);
     if (st) return st;
-    XPBD_CU(c, t.Y.alloc(2 * (size_t)n));
-    XPBD_CU(c, cudaMemcpy(t.Y.p, Y, sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice));
+    st = upload_rows(c, X, Y, n, t);
+    if (st) return st;
     XPBD_CU(c, cudaMemsetAsync(c->mse.p, 0, sizeof(double), c->stream));
-    enqueue_loss_grad(c, t.X.p, t.Y.p, (int)n);
+    enqueue_loss_grad(c, t.X, t.Y, (int)n);
     XPBD_CU(c, cudaGetLastError());
+    // the results through pinned memory, one wait for all of them
+    MlpResults* r = c->h_mlp;
+    XPBD_CU(c, cudaMemcpyAsync(&r->flags, c->flags.p, sizeof r->flags, cudaMemcpyDeviceToHost, c->stream));
+    XPBD_CU(c, cudaMemcpyAsync(&r->loss, c->mse.p, sizeof r->loss, cudaMemcpyDeviceToHost, c->stream));
+    if (grad)
+        XPBD_CU(c, cudaMemcpyAsync(r->grad, c->mlp_g.p, sizeof r->grad, cudaMemcpyDeviceToHost, c->stream));
     XPBD_CU(c, cudaStreamSynchronize(c->stream));
-    st = check_timeouts(c);
-    if (st) return st;
-    if (loss) {
-        double v = 0;
-        XPBD_CU(c, cudaMemcpy(&v, c->mse.p, sizeof v, cudaMemcpyDeviceToHost));
-        *loss = v / (double)n;
-    }
-    if (grad) XPBD_CU(c, cudaMemcpy(grad, c->mlp_g.p, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost));
+    if (r->flags.timeouts)
+        return fail(c, XPBD_ERR_TIMEOUT, "%llu blocks gave up waiting on the tensor cores", r->flags.timeouts);
+    if (loss) *loss = r->loss / (double)n;
+    if (grad) std::memcpy(grad, r->grad, sizeof r->grad);
     return XPBD_OK;
 }
 
