@@ -150,32 +150,46 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
     const int P = (int)pmeta.size(), V = c->V;
     std::vector<int4> tasks;
     std::vector<int> tcol, task_of(P);
-    // Every colour in as many tasks as the largest one needs, each with an equal
-    // share of its patches (both follow the mesh order): the k-th tasks of the
-    // colours then cover the same part of the mesh, also where the colours
-    // differ in size, and a warp mostly waits for its own earlier tasks. (With
-    // runs of 32 the k-th tasks drift apart: per colour of a sweep 3.95 against
-    // 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47 x 49 x 45, the
-    // same for 48 x 48 x 48.)
-    int per_colour = 1;
-    for (int col = 0; col < c->n_tet_colours; col++)
-        per_colour = std::max(per_colour, (c->pcol_off[col + 1] - c->pcol_off[col] + kTaskPatches - 1) / kTaskPatches);
-    for (int col = 0; col < c->n_tet_colours; col++) {
-        const long long first = c->pcol_off[col], count = c->pcol_off[col + 1] - first;
-        for (int i = 0; i < per_colour; i++) {
-            const int q = (int)(first + count * i / per_colour), n = (int)(first + count * (i + 1) / per_colour) - q;
-            int slots = 0;
-            for (int k = 0; k < n; k++) {
-                task_of[q + k] = (int)tasks.size();
-                // the task's tets form one contiguous slot range (bulk-copied whole)
-                if (pmeta[q + k].x != pmeta[q].x + slots)
-                    return fail(c, XPBD_ERR_STATE, "dataflow: patch %d does not continue its task's slots", q + k);
-                slots += pmeta[q + k].y & 0xff;
+    // Within an instance, every colour in as many tasks as the largest one needs,
+    // each with an equal share of its patches (both follow the mesh order): the
+    // k-th tasks of the colours then cover the same part of the mesh, also where
+    // the colours differ in size, and a warp mostly waits for its own earlier
+    // tasks. (With runs of 32 the k-th tasks drift apart: per colour of a sweep
+    // 3.95 against 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47 x 49
+    // x 45, the same for 48 x 48 x 48; shares of the union of 96
+    // uneven instances instead of each one's: 4.17 against 3.99 ms a pass.)
+    const int K = c->n_inst, ncol = c->n_tet_colours;
+    std::vector<int> first((size_t)ncol * (K + 1));  // [colour][instance] first patch
+    std::vector<int> per_colour(K, 1);
+    for (int col = 0; col < ncol; col++) {
+        int q = c->pcol_off[col];
+        for (int k = 0; k <= K; k++) {
+            while (k > 0 && q < c->pcol_off[col + 1] && c->tet_of_slot[pmeta[q].x] < c->toff[k]) q++;
+            first[(size_t)col * (K + 1) + k] = q;
+            if (k > 0) {
+                const int n = q - first[(size_t)col * (K + 1) + k - 1];
+                per_colour[k - 1] = std::max(per_colour[k - 1], (n + kTaskPatches - 1) / kTaskPatches);
             }
-            tasks.push_back(n ? make_int4(q, n, pmeta[q].x, slots) : make_int4(0, 0, 0, 0));
-            tcol.push_back(col);
         }
     }
+    for (int col = 0; col < ncol; col++)
+        for (int k = 0; k < K; k++) {
+            const long long q0 = first[(size_t)col * (K + 1) + k], count = first[(size_t)col * (K + 1) + k + 1] - q0;
+            for (int i = 0; i < per_colour[k]; i++) {
+                const int q = (int)(q0 + count * i / per_colour[k]);
+                const int n = (int)(q0 + count * (i + 1) / per_colour[k]) - q;
+                int slots = 0;
+                for (int j = 0; j < n; j++) {
+                    task_of[q + j] = (int)tasks.size();
+                    // the task's tets form one contiguous slot range (bulk-copied whole)
+                    if (pmeta[q + j].x != pmeta[q].x + slots)
+                        return fail(c, XPBD_ERR_STATE, "dataflow: patch %d does not continue its task's slots", q + j);
+                    slots += pmeta[q + j].y & 0xff;
+                }
+                tasks.push_back(n ? make_int4(q, n, pmeta[q].x, slots) : make_int4(0, 0, 0, 0));
+                tcol.push_back(col);
+            }
+        }
     const int NT = (int)tasks.size();
     auto pv = [&](int q, int k) {
         const int4& a = pverts[2 * (size_t)q + (k >> 2)];
@@ -213,14 +227,13 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
         doff[j + 1] = (int)dep.size();
     }
     const bool staged = c->prm.gs_variant == 3;
-    // variant 4 may fall back to variant 2 (below), so its grid fits both
+    // variant 4 falls back to variant 2 (below) where it needs the lists
     const bool with_faces = c->F > 0;  // variant 4 may then run the contacts inside the sweep
-    const int per_sm =
-        c->prm.gs_variant == 4
-            ? std::min(std::min(sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, false),
-                                with_faces ? sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, true) : 1 << 20),
-                       sweep_dataflow_blocks_per_sm(false, c->prm.gs_min_blocks))
-            : sweep_dataflow_blocks_per_sm(staged, c->prm.gs_min_blocks);
+    int per_sm = lists ? sweep_dataflow_blocks_per_sm(staged, c->prm.gs_min_blocks) : 1 << 20;
+    if (c->prm.gs_variant == 4) {
+        per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, false));
+        if (with_faces) per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, true));
+    }
     int dev = 0, sms = 0;
     XPBD_CU(c, cudaGetDevice(&dev));
     XPBD_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
