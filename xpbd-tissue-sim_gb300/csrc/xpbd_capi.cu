@@ -244,9 +244,19 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     const bool have_faces = c->F > 0, have_static = have_faces && c->static_seen;
     const bool warm = c->warm_mode != XPBD_WARM_NONE;
     const bool cluster = use_cluster(c);
-    // on chip the inertial move is part of the sweep's launch when nothing
-    // reads the predicted positions before it
-    const bool fuse_predict = cluster && cluster_fused(c) && !solve_only && !track && !warm && !c->record;
+    const bool jacobi = p.solver_type == XPBD_SOLVER_JACOBI;
+    // every iteration and colour in one cooperative launch (with faces: the
+    // versioned sweep, static contacts after each iteration's patches)
+    const bool one_launch =
+        !jacobi && !cluster && !separate && !every_iter && c->att_v.empty() &&
+        (!have_faces || (p.gs_variant == 4 && c->flow_versioned && c->flow_contacts && !c->self_on && !c->nbodies)) &&
+        (p.gs_variant == 2 || p.gs_variant == 3 || p.gs_variant == 4) && c->ntasks > 0;
+    const bool versioned = one_launch && p.gs_variant == 4 && c->flow_versioned;
+    // the inertial move is part of the on-chip sweep's launch, or of the
+    // versioned sweep's copy into its records, when nothing reads the predicted
+    // positions before them
+    const bool fuse_predict = ((cluster && cluster_fused(c)) || (versioned && iters > 0)) && !solve_only && !track &&
+                              !warm && !c->record;
     if (!solve_only && !fuse_predict) {
         Scope sc(c, K_PREDICT);
         if (p.first_order) launch_predict_first_order(c->L(), c->x.p, c->prev.p, c->gdz.p, c->V);
@@ -265,7 +275,6 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
         // lambda <- 0 (XPBDSolver.hpp:71-77) before the r(x_pred, 0) evaluation
         if (track) cudaMemsetAsync(c->lam.p, 0, sizeof(float2) * (size_t)c->T, s);
     }
-    const bool jacobi = p.solver_type == XPBD_SOLVER_JACOBI;
     const bool local = !solve_only && have_faces && p.num_local_collision_iters > 0 && c->local_slots.p;
     const bool fuse_final = !track && !local && !solve_only;
     const bool final_on_chip = fuse_predict && fuse_final;
@@ -335,14 +344,8 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
             Scope sc(c, K_PROJECT_GS);
             launch_versions_out(c->L(), c->x.p, c->xv.p, c->vperm.p, c->V);
         }
-    } else if (!separate && !every_iter && c->att_v.empty() &&
-               (!have_faces || (p.gs_variant == 4 && c->flow_versioned && c->flow_contacts && !c->self_on &&
-                                !c->nbodies)) &&
-               (p.gs_variant == 2 || p.gs_variant == 3 || p.gs_variant == 4) && c->ntasks > 0) {
-        // every iteration and colour in one cooperative launch (with faces:
-        // the versioned sweep, static contacts after each iteration's patches)
+    } else if (one_launch) {
         if (track && !warm) exact_residual_row(c, 0, false);
-        const bool versioned = p.gs_variant == 4 && c->flow_versioned;
         if (versioned) {
             // the abort flag (after the epochs, which variant 4 does not use)
             cudaMemsetAsync(c->flow_epoch.p + c->ntasks, 0, sizeof(unsigned), s);
@@ -355,7 +358,9 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
                 have_static ? c->flowc() : xg::FlowContacts{nullptr, nullptr, nullptr, nullptr, nullptr};
             launch_sweep_versioned(c->L(), c->tets(), c->patches_v(), c->patch_ver.p, c->tasks(), iters, !warm, c->x.p,
                                    c->xv.p, c->V, c->vperm.p, c->flags.p, c->flow_grid, p.gs_min_blocks,
-                                   c->flow_resident, ca, fc);
+                                   c->flow_resident, ca, fc,
+                                   xg::ClusterIo{c->x.p, c->prev.p, c->vel.p, p.first_order ? c->gdz.p : nullptr,
+                                                 nullptr, nullptr, dt, dz, fuse_predict, final_on_chip, write_vel});
             c->launches += 2;  // the copies into and out of the versioned positions
         } else
             launch_sweep_dataflow(c->L(), c->tets(), c->patches(), c->tasks(), iters, !warm, c->x.p, c->flags.p,

@@ -1145,6 +1145,39 @@ __global__ void k_versions_out(float4* __restrict__ x, const VerRec* __restrict_
     x[i] = make_float4(ver_val(r.x), ver_val(r.y), ver_val(r.z), x[i].w);
 }
 
+// The inertial move (k_predict, or with gdz k_predict_first_order) straight
+// into the records: x keeps the position before the substep until
+// k_versions_finalize.
+__global__ void k_versions_predict(VerRec* __restrict__ xv, const float4* __restrict__ x, float4* __restrict__ prev,
+                                   const float4* __restrict__ vel, const float* __restrict__ gdz,
+                                   const int* __restrict__ vperm, int V, float dt, float dz) {
+    pdl_wait_then_release();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= V) return;
+    const float4 p = x[i];
+    prev[i] = p;
+    float4 q;
+    if (gdz) {
+        q = make_float4(p.x, p.y, p.z + __ldg(gdz + i), p.w);
+    } else {
+        const float4 v = vel[i];
+        q = make_float4(p.x + dt * v.x, p.y + dt * v.y, (p.z + dt * v.z) + dz, p.w);
+    }
+    xv[vperm[i]] = VerRec{__float_as_uint(q.x), __float_as_uint(q.y), __float_as_uint(q.z), __float_as_uint(q.w)};
+}
+
+// The records back as the substep's result: fixed vertices to prev, velocities.
+__global__ void k_versions_finalize(float4* __restrict__ x, const VerRec* __restrict__ xv,
+                                    const int* __restrict__ vperm, const float4* __restrict__ prev,
+                                    float4* __restrict__ vel, int V, float dt, bool write_vel) {
+    pdl_wait_then_release();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= V) return;
+    const VerRec r = xv[vperm[i]];
+    finalize_vertex(x, prev, vel, i, make_float4(ver_val(r.x), ver_val(r.y), ver_val(r.z), ver_val(r.w)), dt,
+                    write_vel);
+}
+
 // One lane's patch task of k_sweep_versioned after its first polls went out:
 // wait for the vertices still short of their due versions, for the task's
 // bulk-copied records and staged multipliers, project the patch's tets in
@@ -2069,9 +2102,13 @@ void launch_versions_out(const Launch& s, float4* x, const VerRec* xv, const int
 cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const PatchArrays& pa, const int4* pver,
                                    const TaskArrays& ta, int iters, bool first_zero, float4* x, VerRec* xv, int V,
                                    const int* vperm, Flags* flags, int grid, int min_blocks, bool resident,
-                                   const ContactArrays& ca, const FlowContacts& fc) {
+                                   const ContactArrays& ca, const FlowContacts& fc, const ClusterIo& io) {
     if (iters <= 0 || ta.ntasks <= 0) return cudaSuccess;
-    launch_versions_in(s, xv, x, vperm, V);
+    if (io.predict)
+        go(k_versions_predict, nblk(V, 256), 256, s, xv, (const float4*)x, io.prev, (const float4*)io.vel, io.gdz,
+           vperm, V, io.dt, io.dz);
+    else
+        launch_versions_in(s, xv, x, vperm, V);
     const int warps = grid * (kFlowBlock / 32);
     const int per_warp = (ta.ntasks + warps - 1) / warps;
     const bool contacts = fc.task != nullptr;
@@ -2103,7 +2140,11 @@ cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const Pa
 #undef XG_VER_M
 #undef XG_VER
     if (e != cudaSuccess) return e;
-    launch_versions_out(s, x, xv, vperm, V);
+    if (io.finalize)
+        go(k_versions_finalize, nblk(V, 256), 256, s, x, (const VerRec*)xv, vperm, (const float4*)io.prev, io.vel, V,
+           io.dt, io.write_vel != 0);
+    else
+        launch_versions_out(s, x, xv, vperm, V);
     return cudaSuccess;
 }
 

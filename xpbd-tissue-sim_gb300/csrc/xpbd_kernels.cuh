@@ -219,6 +219,7 @@ struct ClusterShape {
     int resident;                      // 1: every record stays in shared memory; 0: two buffers, one colour each
     size_t smem;
 };
+// what a one-launch sweep does around its iterations
 struct ClusterIo {
     float4 *x, *prev, *vel;
     const float* gdz;   // first order: the inertial z move (else nullptr)
@@ -357,13 +358,16 @@ int sweep_dataflow_blocks_per_sm(bool staged, int min_blocks);
 // shared memory (ntasks / warps <= kResidentTasks; sweep_versioned_smem bytes
 // per block).
 // fc.task != nullptr: the static contacts of ca run inside the sweep (FlowContacts).
+// io.predict, io.finalize: the inertial move on the way in (x then keeps the
+// position before the substep), the fixed reset and velocities on the way out
+// (only together with io.predict).
 // The sweep numbers the vertices its own way (vperm: vertex -> record of xv,
 // chosen so that a task's lanes touch neighbouring records); pa.verts and
 // fc.vfaces are in that numbering.
 cudaError_t launch_sweep_versioned(const Launch& s, const TetArrays& t, const PatchArrays& pa, const int4* pver,
                                    const TaskArrays& ta, int iters, bool first_zero, float4* x, VerRec* xv, int V,
                                    const int* vperm, Flags* flags, int grid, int min_blocks, bool resident,
-                                   const ContactArrays& ca, const FlowContacts& fc);
+                                   const ContactArrays& ca, const FlowContacts& fc, const ClusterIo& io);
 // blocks per SM of the versioned sweep with the dynamic shared memory it
 // needs when each warp owns `tasks_per_warp` tasks (0: not resident), with or
 // without the contact phases
