@@ -74,7 +74,7 @@ def workload(name, solver=None, mesher=None):
 def describe(w, jacobi_variant=0):
     import workloads as W
     solver = "coloured Gauss-Seidel" if w.solver == W.GAUSS_SEIDEL else \
-        ("Jacobi (per-tet deltas + CSR gather)" if jacobi_variant == 1 else "Jacobi (vector atomics)")
+        ("Jacobi (block partial sums + gather)" if jacobi_variant == 1 else "Jacobi (vector atomics)")
     d = {
         "workload": f"{w.name}: {w.T:,} tets, {w.V:,} vertices",
         "solver": solver,
@@ -939,7 +939,7 @@ def main():
     ap.add_argument("--min-blocks", type=int, default=0, choices=[0, 6, 8], help="patch kernel blocks/SM target")
     ap.add_argument("--variant", type=int, default=None, choices=[0, 1, 2, 3, 4], help="Gauss-Seidel sweep kernel variant")
     ap.add_argument("--jacobi-variant", type=int, default=None, choices=[0, 1],
-                    help="Jacobi: 0 vector atomics, 1 per-tet deltas + CSR gather")
+                    help="Jacobi: 0 vector atomics, 1 block partial sums + gather")
     ap.add_argument("--poll-ns", type=int, default=0, help="versioned sweep: back-off between polls (ns)")
     ap.add_argument("--topology-reload", action="store_true",
                     help="versioned sweep: reload task topology every phase")

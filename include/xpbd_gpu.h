@@ -58,7 +58,7 @@ extern "C" {
 
 /* Jacobi scatter variant */
 #define XPBD_JACOBI_ATOMIC 0   /* warp-level vector atomics into a delta buffer  */
-#define XPBD_JACOBI_GATHER 1   /* per-tet deltas + vertex->tet CSR gather        */
+#define XPBD_JACOBI_GATHER 1   /* partial sums per block of tets, then a gather  */
 
 typedef struct xpbd_ctx xpbd_ctx;
 
@@ -106,6 +106,7 @@ typedef struct {
                                /* (else as 1); 4 dataflow on version-stamped       */
                                /* vertices: a patch polls the versions of its own  */
                                /* vertices, no task counters or fences (else as 0);*/
+                               /* small meshes on chip, one cluster an instance;   */
                                /* default 4                                        */
     int32_t num_local_collision_iters; /* num-local-collision-iters: passes    */
                                /* after the global solve over every contact    */
