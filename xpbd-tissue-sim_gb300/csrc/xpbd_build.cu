@@ -21,6 +21,7 @@
 #include "xpbd_ctx.cuh"
 #include "xpbd_host.cuh"
 #include "xpbd_kernels.cuh"
+#include "xpbd_partition.hpp"
 
 using namespace xg;
 
@@ -480,15 +481,22 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         const int kk = k & 3;
         return kk == 0 ? a.x : (kk == 1 ? a.y : (kk == 2 ? a.z : a.w));
     };
-    // each instance's patches, their rest centroids
-    std::vector<std::vector<int>> mine(K);
-    std::vector<double> centre(3 * (size_t)P, 0.0);
+    PatchSet ps;
+    ps.V = V; ps.K = K; ps.ncol = ncol; ps.per = kMaxPatchVerts;
+    ps.vert.assign((size_t)P * kMaxPatchVerts, -1);
+    ps.colour.resize(P);
+    ps.mine.resize(K);
+    ps.centre.assign(3 * (size_t)P, 0.0);
+    for (int col = 0; col < ncol; col++)
+        for (int q = c->pcol_off[col]; q < c->pcol_off[col + 1]; q++) ps.colour[q] = col;
     for (int q = 0; q < P; q++) {
         const int64_t t = c->tet_of_slot[pmeta[q].x];
-        mine[std::upper_bound(c->toff.begin(), c->toff.end(), t) - c->toff.begin() - 1].push_back(q);
+        ps.mine[std::upper_bound(c->toff.begin(), c->toff.end(), t) - c->toff.begin() - 1].push_back(q);
         const int n = pmeta[q].y >> 8;
-        for (int k = 0; k < n; k++)
-            for (int i = 0; i < 3; i++) centre[3 * (size_t)q + i] += X[3 * (size_t)pv(q, k) + i] / n;
+        for (int k = 0; k < n; k++) {
+            ps.vert[(size_t)q * kMaxPatchVerts + k] = pv(q, k);
+            for (int i = 0; i < 3; i++) ps.centre[3 * (size_t)q + i] += X[3 * (size_t)pv(q, k) + i] / n;
+        }
     }
     // per patch and vertex slot the patches around the vertex and those of a
     // lower colour (slot order is colour order, and a colour holds a vertex once)
@@ -514,121 +522,22 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         for (int k = 0; k < kMaxPatchVerts; k++)
             for (int q = q0; q < std::min(P, q0 + 32); q++)
                 if (k < (pmeta[q].y >> 8) && rank[pv(q, k)] < 0) rank[pv(q, k)] = ranks++;
-    // pieces of [first, last) of an instance's patches into blocks b .. b + n - 1
-    std::vector<int> block(P, 0);
-    auto bisect = [&](auto&& self, std::vector<int>& list, size_t first, size_t last, int b, int n) -> void {
-        if (n == 1) {
-            for (size_t i = first; i < last; i++) block[list[i]] = b;
-            return;
-        }
-        double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-        for (size_t i = first; i < last; i++)
-            for (int k = 0; k < 3; k++) {
-                lo[k] = std::min(lo[k], centre[3 * (size_t)list[i] + k]);
-                hi[k] = std::max(hi[k], centre[3 * (size_t)list[i] + k]);
-            }
-        int ax = 0;
-        for (int k = 1; k < 3; k++)
-            if (hi[k] - lo[k] > hi[ax] - lo[ax]) ax = k;
-        const size_t mid = first + (last - first) / 2;
-        std::nth_element(list.begin() + first, list.begin() + mid, list.begin() + last, [&](int a, int d) {
-            const double u = centre[3 * (size_t)a + ax], v = centre[3 * (size_t)d + ax];
-            return u < v || (u == v && a < d);
-        });
-        self(self, list, first, mid, b, n / 2);
-        self(self, list, mid, last, b + n / 2, n / 2);
-    };
-    std::vector<int> pcol(P);
-    for (int col = 0; col < ncol; col++)
-        for (int q = c->pcol_off[col]; q < c->pcol_off[col + 1]; q++) pcol[q] = col;
-    // n slabs across axis ax, the cuts moved to the nearest step of the
-    // coordinate (a layer of a grid) within half a slab
-    std::vector<std::vector<int>> by_axis[3];
-    auto slabs = [&](int ax, int n) {
-        auto at = [&](int q) { return centre[3 * (size_t)q + ax]; };
-        if (by_axis[ax].empty()) {
-            by_axis[ax] = mine;
-            for (auto& l : by_axis[ax])
-                std::sort(l.begin(), l.end(), [&](int a, int d) { return at(a) < at(d) || (at(a) == at(d) && a < d); });
-        }
-        for (int k = 0; k < K; k++) {
-            const std::vector<int>& l = by_axis[ax][k];
-            const long long m = (long long)l.size();
-            const double eps = 1e-6 * (at(l.back()) - at(l.front()));
-            long long lo = 0;
-            for (int r = 0; r < n; r++) {
-                long long hi = m * (r + 1) / n;
-                for (long long d = 0; r + 1 < n && 2 * n * d <= m; d++) {
-                    const long long up = hi + d, down = hi - d;
-                    if (up < m && at(l[up]) - at(l[up - 1]) > eps) { hi = up; break; }
-                    if (down > lo && at(l[down]) - at(l[down - 1]) > eps) { hi = down; break; }
-                }
-                for (long long i = lo; i < hi; i++) block[l[i]] = k * n + r;
-                lo = std::max(lo, hi);
-            }
-        }
-    };
-    // shape 0-2: slabs across that axis; 3: recursive bisection (n a power of two)
-    std::vector<int> cnt;
-    auto assign = [&](int shape, int n) {  // -> the most patches of one colour in a block
-        if (shape < 3) slabs(shape, n);
-        else for (int k = 0; k < K; k++) bisect(bisect, mine[k], 0, mine[k].size(), k * n, n);
-        cnt.assign((size_t)K * n * ncol, 0);
-        int worst = 0;
-        for (int q = 0; q < P; q++) worst = std::max(worst, ++cnt[(size_t)block[q] * ncol + pcol[q]]);
-        return worst;
-    };
-    // colours with a vertex that another block wrote in the colour before: their
-    // phases wait for it (about 0.75 us on GB300; a write two phases back is there)
-    auto stalls = [&]() {
-        std::vector<int> first(V, -1), last(V, -1);
-        std::vector<char> s(ncol, 0);
-        for (int q = 0; q < P; q++)
-            for (int k = 0; k < (pmeta[q].y >> 8); k++) {
-                const int v = pv(q, k), l = last[v];
-                if (l < 0) first[v] = q;
-                else if (block[l] != block[q] && pcol[l] + 1 == pcol[q]) s[pcol[q]] = 1;
-                last[v] = q;
-            }
-        for (int v = 0; v < V; v++)
-            if (last[v] >= 0 && pcol[first[v]] == 0 && pcol[last[v]] == ncol - 1 && block[first[v]] != block[last[v]])
-                s[0] = 1;
-        return (int)std::count(s.begin(), s.end(), 1);
-    };
-    size_t largest = 0;
-    for (int k = 0; k < K; k++) largest = std::max(largest, mine[k].size());
-    struct Choice {
-        double us;
-        int n, shape;
-    };
-    std::vector<Choice> choices;
+    ClusterPartition part_of(ps);
+    const std::vector<int>& block = part_of.block;
+    std::vector<int> cnt, pcol;
     const double other = separate ? 2.9 : 2.2;
-    const int n_min = (int)std::min<size_t>(kMaxClusterSize, (largest + kClusterLanes * ncol - 1) / (kClusterLanes * ncol));
-    for (int n : {n_min, n_min + 1, n_min + 2, n_min + 4, kMaxClusterSize}) {
-        // self-collisions take their own launches between the sweeps: one block only
-        if (n > kMaxClusterSize || (n > 1 && c->prm.self_collisions) || (K > 1 && K * n > sms) || (!choices.empty() && choices.back().n == n)) continue;
-        for (int sh = 0; sh < 4; sh++) {
-            if ((n == 1 && sh > 0) || (sh == 3 && (n & (n - 1)))) continue;
-            assign(sh, n);
-            double us = 0;
-            for (int col = 0; col < ncol; col++) {
-                int most = 1;
-                for (int b = 0; b < K * n; b++) most = std::max(most, cnt[(size_t)b * ncol + col]);
-                us += (n == 1 ? (separate ? 1.65 : 1.1) : (separate ? 2.2 : 1.4)) *
-                      ((most + kClusterLanes - 1) / kClusterLanes);
-            }
-            if (us < other * ncol && n > 1) us += 0.75 * stalls();
-            choices.push_back(Choice{us, n, sh});
-        }
-    }
-    std::stable_sort(choices.begin(), choices.end(), [](const Choice& a, const Choice& b) { return a.us < b.us; });
+    // self-collisions take their own launches between the sweeps: one block only
+    const std::vector<ClusterChoice> choices =
+        part_of.choices(kClusterLanes, kMaxClusterSize, sms, c->prm.self_collisions != 0, separate ? 1.65 : 1.1,
+                        separate ? 2.2 : 1.4, other);
     const int colours = ncol;
-    const std::vector<int> colour_of = pcol;
-    for (const Choice& ch : choices) {
+    const std::vector<int>& colour_of = ps.colour;
+    for (const ClusterChoice& ch : choices) {
         if (ch.us >= other * colours) break;
         ncol = colours;
         pcol = colour_of;
-        assign(ch.shape, ch.n);
+        part_of.assign(ch.shape, ch.n);
+        cnt = part_of.count;
         const int csize = ch.n, ncta = K * csize;
         {
             // rounds: the i-th of a block's n patches of a colour in round i * rounds / n
