@@ -11,6 +11,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PROGRAM = r"""
 #include <cstdio>
 #include <cstdlib>
+#include <random>
 #include "xpbd_partition.hpp"
 using namespace xg::host;
 
@@ -41,9 +42,54 @@ static PatchSet grid(int K, int nx, int ny, int nz) {
     return s;
 }
 
+// n patches of up to eight of the vertices around a random point, coloured greedily
+static PatchSet cloud(int n) {
+    PatchSet s;
+    s.K = 1; s.V = 2 * n;
+    std::mt19937 rng(5);
+    std::uniform_real_distribution<double> u(0.0, 1.0);
+    std::vector<double> X(3 * s.V);
+    for (double& x : X) x = u(rng);
+    std::vector<std::vector<int>> items(n);
+    std::vector<double> at(3 * n);
+    std::vector<int> col(n), order(s.V);
+    std::vector<std::vector<char>> used(s.V, std::vector<char>(256, 0));
+    for (int q = 0; q < n; q++) {
+        for (int k = 0; k < 3; k++) at[3 * q + k] = u(rng);
+        for (int v = 0; v < s.V; v++) order[v] = v;
+        auto dist = [&](int v) {
+            double d = 0;
+            for (int k = 0; k < 3; k++) d += (X[3 * v + k] - at[3 * q + k]) * (X[3 * v + k] - at[3 * q + k]);
+            return d;
+        };
+        const int m = 4 + q % 5;
+        std::partial_sort(order.begin(), order.begin() + m, order.end(), [&](int a, int b) { return dist(a) < dist(b); });
+        items[q].assign(order.begin(), order.begin() + m);
+        int c = 0;
+        for (bool again = true; again;) {
+            again = false;
+            for (int v : items[q]) again = again || used[v][c];
+            if (again) c++;
+        }
+        for (int v : items[q]) used[v][c] = 1;
+        col[q] = c;
+        s.ncol = std::max(s.ncol, c + 1);
+    }
+    s.mine.resize(1);
+    for (int c = 0; c < s.ncol; c++)
+        for (int q = 0; q < n; q++) {
+            if (col[q] != c) continue;
+            s.mine[0].push_back((int)s.colour.size());
+            s.colour.push_back(c);
+            for (int k = 0; k < 8; k++) s.vert.push_back(k < (int)items[q].size() ? items[q][k] : -1);
+            for (int k = 0; k < 3; k++) s.centre.push_back(at[3 * q + k]);
+        }
+    return s;
+}
+
 int main(int argc, char** argv) {
     const int K = std::atoi(argv[1]), nx = std::atoi(argv[2]), ny = std::atoi(argv[3]), nz = std::atoi(argv[4]);
-    const PatchSet s = grid(K, nx, ny, nz);
+    const PatchSet s = K ? grid(K, nx, ny, nz) : cloud(nx);
     ClusterPartition p(s);
     for (int n = 1; n <= 16; n++)
         for (int shape = 0; shape < 4; shape++) {
@@ -54,8 +100,18 @@ int main(int argc, char** argv) {
                     if (p.block[q] < k * n || p.block[q] >= (k + 1) * n) return 1;
             p.stalls();
         }
-    for (const ClusterChoice& c : p.choices(128, 16, 152, false, 1.1, 1.4, 2.2))
-        std::printf("%d %d %.2f\n", c.n, c.shape, c.us);
+    for (const ClusterChoice& c : p.choices(128, 16, 152, false, 1.1, 1.4, 2.2)) {
+        p.assign(c.shape, c.n);
+        size_t most = 0;  // blocks that hold one vertex
+        std::vector<std::vector<int>> in(s.V);
+        for (int q = 0; q < s.patches(); q++)
+            for (int k = 0; k < 8 && s.vert[8 * (size_t)q + k] >= 0; k++) {
+                std::vector<int>& l = in[s.vert[8 * (size_t)q + k]];
+                if (std::find(l.begin(), l.end(), p.block[q]) == l.end()) l.push_back(p.block[q]);
+                most = std::max(most, l.size());
+            }
+        std::printf("%d %d %.2f %zu\n", c.n, c.shape, c.us, most);
+    }
     return 0;
 }
 """
@@ -78,3 +134,18 @@ def test_partition_of_fewer_patches_than_blocks(planner, K, dims):
     blocks reads inside its lists and keeps each instance in its own blocks."""
     r = subprocess.run([planner, str(K), *map(str, dims)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("K,dims", [(1, (24, 24, 24)), (1, (20, 35, 20)), (1, (19, 33, 19)), (1, (10, 100, 10)),
+                                    (1, (20, 20, 20)), (1, (1, 40, 1)), (7, (10, 10, 10)), (5, (14, 14, 14)),
+                                    (0, (1500, 0, 0)), (0, (4000, 0, 0))])
+def test_no_vertex_lies_in_more_than_two_blocks(planner, K, dims):
+    """A vertex's copies are written without a fence between the blocks, which
+    keeps its versions in order for two holders and not for three. K = 0: an
+    unstructured set of patches."""
+    r = subprocess.run([planner, str(K), *map(str, dims)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    rows = [line.split() for line in r.stdout.splitlines()]
+    assert all(int(most) <= 2 for _, _, _, most in rows), rows
+    if K == 1 and dims == (10, 100, 10):  # the beam keeps its slabs
+        assert rows[0][:2] == ["10", "1"]

@@ -572,8 +572,8 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         std::vector<int4> vers(P);
         std::vector<float4> recs(3 * (size_t)c->T);
         int nrec = 0;
-        // the blocks' vertices: which of them hold each vertex (at most nine)
-        constexpr int kCopies = 9;
+        // the blocks' vertices: which of them hold each vertex (two at most, as choices() sees to)
+        constexpr int kCopies = 2;
         std::vector<int> copy((size_t)V * kCopies, -1), copies(V, 0), local((size_t)V * kCopies, 0);
         bool ok = true;
         for (int q = 0; q < P && ok; q++)
@@ -593,7 +593,7 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
             return (size_t)v * kCopies + j;
         };
         std::vector<int> verts;
-        std::vector<uint4> remote;
+        std::vector<unsigned> remote;
         std::vector<char> seen(V, 0);  // per block: 1 numbered
         bool generic = false;
         size_t max_rec = 0;
@@ -665,13 +665,12 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         for (int b = 0; b < ncta; b++)
             for (int i = 0; i < part[2 * b].z; i++) {
                 const int v = verts[part[2 * b].x + i] & 0x7fffffff;
-                unsigned short r[kCopies - 1];
-                std::fill(r, r + kCopies - 1, (unsigned short)0xffff);
-                for (int j = 0, n = 0; j < copies[v]; j++) {
+                for (int j = 0; j < copies[v]; j++) {
                     const int o = copy[(size_t)v * kCopies + j];
-                    if (o != b) r[n++] = (unsigned short)((o % csize) << 12 | local[(size_t)v * kCopies + j]);
+                    if (o != b)
+                        remote[part[2 * b + 1].y + i] =
+                            (unsigned)(o % csize) << 12 | (unsigned)local[(size_t)v * kCopies + j];
                 }
-                std::memcpy(&remote[part[2 * b + 1].y + i], r, sizeof(uint4));
             }
         // what each colour sends to the other blocks
         std::vector<uint2> send;
@@ -709,7 +708,7 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         s.max_t = (s.max_t + 1) / 2 * 2;
         s.max_nb = (s.max_nb + 3) / 4 * 4;
         const size_t rest = 16 * (size_t)s.max_nv + (csize > 1 ? 48 : 32) * (size_t)s.max_p +
-                            (csize > 1 ? 28 : 0) * (size_t)s.max_nb + 8 * (size_t)s.max_send + 8 * (size_t)s.max_t + (generic ? 16 * (size_t)kMaxPatchVerts * kClusterLanes : 0);
+                            (csize > 1 ? 16 : 0) * (size_t)s.max_nb + 8 * (size_t)s.max_send + 8 * (size_t)s.max_t + (generic ? 16 * (size_t)kMaxPatchVerts * kClusterLanes : 0);
         const size_t all = 48 * (size_t)s.max_t, two = 2 * 48 * max_rec;
         s.resident = rest + all <= (size_t)kClusterSmemMax;
         s.rec_cap = (int)(s.resident ? (size_t)s.max_t : max_rec);
@@ -751,7 +750,7 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         const size_t o_range = put(range.data(), sizeof(int4) * range.size());
         const size_t o_vidx = put(vidx.data(), sizeof(int4) * vidx.size());
         const size_t o_meta = put(meta.data(), sizeof(int4) * meta.size());
-        const size_t o_rem = put(remote.data(), sizeof(uint4) * remote.size());
+        const size_t o_rem = put(remote.data(), sizeof(unsigned) * remote.size());
         const size_t o_face = put(fl.data(), sizeof(int4) * fl.size());
         const size_t o_vert = put(verts.data(), sizeof(int) * verts.size());
         const size_t o_slot = put(slots.data(), sizeof(int) * slots.size());
@@ -764,7 +763,7 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         const int4* d = c->cl_tab.p;
         c->cl = ClusterArrays{d + o_part, d + o_range, d + o_vidx, d + o_meta, d + o_ver, (const int*)(d + o_slot),
                               (const float4*)(d + o_rec), (size_t)c->T, (const int*)(d + o_vert),
-                              (const uint4*)(d + o_rem), (const uint2*)(d + o_send), (const int*)(d + o_soff),
+                              (const unsigned*)(d + o_rem), (const uint2*)(d + o_send), (const int*)(d + o_soff),
                               d + o_face, nullptr, nullptr};
         c->cl_shape = s;
         c->cluster_on = true;

@@ -1,9 +1,8 @@
 // Gauss-Seidel on chip: a whole substep of a small mesh in one launch of one
 // thread-block cluster per instance. Vertices, multipliers and the patches'
 // topology live in shared memory for the whole solve, a colour ends at a
-// cluster (or, with one block, a block) barrier, and a vertex that several
-// blocks hold is written into each of their copies over distributed shared
-// memory. Same patches, colours, order and arithmetic as the colour launches
+// cluster (or, with one block, a block) barrier, and a vertex that two blocks
+// hold is written into the other's copy over distributed shared memory. Same patches, colours, order and arithmetic as the colour launches
 // and the versioned sweep (xpbd_kernels.cu); the results agree bit for bit.
 //
 // Measured on GB300, per substep against the versioned sweep with its launches
@@ -30,7 +29,7 @@ __device__ __forceinline__ unsigned mapa(unsigned addr, unsigned rank) {
 }
 
 // A block's vertex: the position and a fourth word in one 128-bit word. The
-// first nb vertices of a block are held by other blocks of the cluster too;
+// first nb vertices of a block are held by one other block of the cluster too;
 // their fourth word is the vertex's version, and the inverse mass, which no
 // sweep changes, lies beside (sw). The others' is the inverse mass. Shared
 // vertices are read and written by one scalar .b128 access, which the PTX
@@ -73,7 +72,7 @@ template <bool MULTI>
 struct BlockVerts {
     VertWord* sv;
     const float* sw;   // [nb] the shared vertices' inverse masses
-    const uint4* rem;  // [nb] their up to eight other copies, 16 bits each: rank << 12 | index, 0xffff = none
+    const unsigned* rem;  // [nb] their other copy: rank << 12 | index
     int nb;
     __device__ __forceinline__ bool shared(int l) const { return MULTI && l < nb; }
     // vertex l into p; whether it is due (a block's own vertices always are)
@@ -94,17 +93,12 @@ struct BlockVerts {
         else st_vert(sv + l, VertWord{pack2(p.x, __float_as_uint(p.y)),
                                       pack2(p.z, shared(l) ? (unsigned)ver : __float_as_uint(p.w))});
     }
-    // a shared vertex into its other copies
+    // a shared vertex into its other copy
     __device__ __forceinline__ void send(int l) const {
         if (!shared(l)) return;
         const VertWord v = ld_vert(sv + l);
-        const uint4 r = rem[l];
-        const unsigned c[4] = {r.x, r.y, r.z, r.w};
-        for (int k = 0; k < 8; k++) {
-            const unsigned m = (c[k >> 1] >> (16 * (k & 1))) & 0xffffu;
-            if (m == 0xffffu) break;
-            st_vert_cluster(mapa(smem_u32(sv) + 16u * (m & 0xfffu), m >> 12), v);
-        }
+        const unsigned m = rem[l];
+        st_vert_cluster(mapa(smem_u32(sv) + 16u * (m & 0xfffu), m >> 12), v);
     }
 };
 
@@ -260,16 +254,22 @@ __device__ __forceinline__ bool cluster_patch(const TetArrays& t, const BlockVer
 // positions and multipliers in and out. The colours here are those of
 // build_cluster, which halves a colour that has more patches than lanes.
 // A phase ends at a barrier of those warps. With several blocks (MULTI) that
-// barrier stays inside the block; a vertex that several hold carries a
+// barrier stays inside the block; a vertex that two blocks hold carries a
 // version, and its readers poll their own copy until the version is due (the
 // versioned sweep's rule: per iteration one version for each patch, and each
 // face with active contacts, around the vertex). Warps 5-7 send what a
-// colour wrote to the other copies, by distributed-shared-memory stores, while the
+// colour wrote to the other copy, by distributed-shared-memory stores, while the
 // next colour is projected. Each version goes out at most once, by its own
 // colour: a vertex that the next colour has already moved on is left to that
-// colour (this block was its next writer, so no other block waits for the
-// version in between), because a second send of one version could land on a
+// colour (this block was its next writer, so the other block does not wait for
+// the version in between), because a second send of one version could land on a
 // newer one that the receiver has written since.
+// No vertex lies in more than two blocks (ClusterPartition::crowded), and that
+// is what orders a copy's versions without a fence: it is written by its own
+// block and by one other. The own block writes version n + 1 after it read n
+// from the copy itself, or wrote n; the other's sends are ordered among
+// themselves by its phase barriers. With a third block, A's store of n into C
+// and B's of n + 1 (made after A's store of n into B) would race.
 template <bool SEPARATE, bool CONTACTS, bool MULTI>
 __global__ void __launch_bounds__(kClusterThreads, 1)
     k_sweep_cluster(ClusterArrays a, ClusterShape s, TetArrays t, ClusterIo io, int iters, bool first_zero,
@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     int4* tv = reinterpret_cast<int4*>(rec + (s.resident ? 3 : 6) * (size_t)s.rec_cap);
     int4* tm = tv + s.max_p;
     int4* td = tm + s.max_p;  // MULTI
-    uint4* rem = reinterpret_cast<uint4*>(td + (MULTI ? s.max_p : 0));
-    unsigned long long* smask = reinterpret_cast<unsigned long long*>(rem + s.max_nb);  // MULTI, CONTACTS
+    unsigned* rem = reinterpret_cast<unsigned*>(td + (MULTI ? s.max_p : 0));  // MULTI
+    unsigned long long* smask = reinterpret_cast<unsigned long long*>(rem + (MULTI ? s.max_nb : 0));  // MULTI, CONTACTS
     float* sw = reinterpret_cast<float*>(smask + (MULTI ? s.max_nb : 0));  // MULTI
     uint2* ssend = reinterpret_cast<uint2*>(sw + (MULTI ? s.max_nb : 0));  // MULTI
     float2* slam = reinterpret_cast<float2*>(ssend + (MULTI ? s.max_send : 0));
@@ -305,18 +305,19 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         mbar_init(&tbar, 1);
-        const unsigned bytes = 16u * (unsigned)((MULTI ? 3 : 2) * np + nb);
+        const unsigned bytes = 16u * (unsigned)((MULTI ? 3 : 2) * np);
         mbar_arrive_expect_tx(&tbar, bytes);
         if (np) {
             tma_load_1d(tv, a.vidx + p0, 16u * (unsigned)np, &tbar);
             tma_load_1d(tm, a.meta + p0, 16u * (unsigned)np, &tbar);
             if (MULTI) tma_load_1d(td, a.ver + p0, 16u * (unsigned)np, &tbar);
         }
-        if (nb) tma_load_1d(rem, a.remote + b0, 16u * (unsigned)nb, &tbar);
     }
     __syncthreads();
-    if (MULTI)
+    if (MULTI) {
+        for (int i = tid; i < nb; i += nt) rem[i] = __ldg(a.remote + b0 + i);
         for (int i = tid; i < ssoff[s.ncol] - ssoff[0]; i += nt) ssend[i] = __ldg(a.send + ssoff[0] + i);
+    }
     int nne = 0;  // colours with patches here, in order
     for (int c = 0; c < s.ncol; c++) {
         if (srg[c].y > 0) {
@@ -411,13 +412,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                         if (l[q] >= nb) continue;
                         const unsigned at = smem_u32(smask) + 4u * (unsigned)(c >> 5), bit = 1u << (c & 31);
                         red_or_cluster(mapa(at + 8u * (unsigned)l[q], blockIdx.x % s.csize), bit);
-                        const uint4 r = rem[l[q]];
-                        const unsigned cp[4] = {r.x, r.y, r.z, r.w};
-                        for (int k = 0; k < 8; k++) {
-                            const unsigned m = (cp[k >> 1] >> (16 * (k & 1))) & 0xffffu;
-                            if (m == 0xffffu) break;
-                            red_or_cluster(mapa(at + 8u * (m & 0xfffu), m >> 12), bit);
-                        }
+                        const unsigned m = rem[l[q]];
+                        red_or_cluster(mapa(at + 8u * (m & 0xfffu), m >> 12), bit);
                     }
                 }
         }

@@ -191,7 +191,7 @@ constexpr unsigned kClusterPolls = 1u << 20;  // polls of a shared vertex before
 constexpr int kMaxClusterColours = 64;   // patch colours, as build_cluster splits them
 constexpr int kClusterSmemMax = 230400;  // dynamic shared memory of a block (227 KB less the static part)
 struct ClusterArrays {
-    const int4* part;       // [2 ncta] (first entry of verts, vertices, of these held by other blocks too,
+    const int4* part;       // [2 ncta] (first entry of verts, vertices, of these held by another block too,
                             //  first entry of vidx / meta / ver / slot), (patches, first entry of remote, tets,
                             //  first tet of rec)
     const int4* range;      // [ncta ncol] (first patch in the block, patches, tets, first tet in the block)
@@ -202,8 +202,7 @@ struct ClusterArrays {
     const float4* rec;      // [3][nrec] the tet records m0, m1, m2 by block, colour, patch
     size_t nrec;
     const int* verts;       // block-local vertex -> vertex, sign bit set in the block that writes it back
-    const uint4* remote;    // the shared vertices' other copies, 8 x 16 bits: block in the cluster << 12 |
-                            // local index, 0xffff = none
+    const unsigned* remote; // the shared vertices' other copy: block in the cluster << 12 | local index
     const uint2* send;      // by block and colour: the shared vertices the colour writes and where to: (local index
                             // << 16 | block in the cluster << 12 | index there, the vertex's 16 bits of ver)
     const int* send_off;    // [ncta (ncol + 1)] its ranges

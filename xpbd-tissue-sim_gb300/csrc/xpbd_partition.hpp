@@ -63,7 +63,24 @@ public:
         return (int)std::count(w.begin(), w.end(), 1);
     }
 
-    // The divisions that may pay, best first. Per round of at most `lanes`
+    // Whether some vertex lies in more than two blocks. Between two blocks the
+    // versions of a vertex alternate, and a block's copy takes them in order:
+    // its own writes follow its reads of the other's. A third block's copy would
+    // be written by two others, and nothing orders their stores.
+    bool crowded() const {
+        std::vector<int> one(s.V, -1), two(s.V, -1);
+        for (int q = 0; q < s.patches(); q++)
+            for (int k = 0; k < s.per && vert(q, k) >= 0; k++) {
+                const int v = vert(q, k), b = block[q];
+                if (one[v] < 0) one[v] = b;
+                else if (one[v] == b || two[v] == b) continue;
+                else if (two[v] < 0) two[v] = b;
+                else return true;
+            }
+        return false;
+    }
+
+    // The divisions that may pay and hold a vertex in two blocks at most, best first. Per round of at most `lanes`
     // patches a block and colour a sweep takes `one` us with one block, `more`
     // with several (and 0.75 where it waits for another block); `other` us a
     // colour is what the route it stands in for takes. most: blocks of a cluster
@@ -75,12 +92,15 @@ public:
         const size_t unit = (size_t)lanes * s.ncol;
         const int n_min = (int)std::min<size_t>(most, (largest + unit - 1) / unit);
         std::vector<ClusterChoice> out;
+        int before = 0;
         for (int n : {n_min, n_min + 1, n_min + 2, n_min + 4, most}) {
-            if (n > most || (n > 1 && single) || (s.K > 1 && s.K * n > sms) || (!out.empty() && out.back().n == n))
+            if (n > most || (n > 1 && single) || (s.K > 1 && s.K * n > sms) || n == before)
                 continue;
+            before = n;
             for (int shape = 0; shape < 4; shape++) {
                 if ((n == 1 && shape > 0) || (shape == 3 && (n & (n - 1)))) continue;
                 assign(shape, n);
+                if (n > 2 && crowded()) continue;
                 double us = 0;
                 for (int col = 0; col < s.ncol; col++) {
                     int worst = 1;
