@@ -354,6 +354,10 @@ int xpbd_health(xpbd_ctx* ctx, int64_t* nonfinite, int64_t* degenerate);
  * tables and the default limit back. XPBD_ERR_STATE without the versioned
  * sweep. Stalls no GPU: every wait is bounded and the kernel returns. */
 int xpbd_debug_stall_vertex(xpbd_ctx* ctx, int32_t vertex, int32_t poll_limit);
+/* The same for the on-chip sweep of several blocks (small meshes, gs_variant
+ * 4): the waits for a vertex that two blocks hold run out. XPBD_ERR_STATE where
+ * the context has no such sweep, or the vertex lies in one block. */
+int xpbd_debug_stall_on_chip(xpbd_ctx* ctx, int32_t vertex, int32_t poll_limit);
 /* Colouring in use (coloured Gauss-Seidel). Tets are grouped into patches
  * (runs of up to gs_patch_tets consecutive tets on at most 8 vertices) and the
  * patches are coloured so that patches of one colour share no vertex; each

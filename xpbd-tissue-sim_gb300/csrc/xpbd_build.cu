@@ -567,6 +567,7 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         ClusterShape s{};
         s.ncta = ncta; s.csize = csize; s.ncol = ncol; s.nfcol = c->n_face_colours;
         s.threads = kClusterThreads;
+        s.polls = kClusterPolls;
         std::vector<int4> part(2 * (size_t)ncta), range((size_t)ncta * ncol), vidx(P), meta(P);
         std::vector<int> slots(P);
         std::vector<int4> vers(P);

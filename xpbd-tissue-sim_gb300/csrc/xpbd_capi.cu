@@ -1501,6 +1501,45 @@ int xpbd_debug_stall_vertex(xpbd_ctx* c, int32_t vertex, int32_t poll_limit) {
     return XPBD_OK;
 }
 
+int xpbd_debug_stall_on_chip(xpbd_ctx* c, int32_t vertex, int32_t poll_limit) {
+    if (!c) return XPBD_ERR_INVALID;
+    if (!c->cluster_on || c->cl_shape.csize < 2)
+        return fail(c, XPBD_ERR_STATE, "no on-chip sweep of several blocks in this context");
+    if (vertex >= c->V || (vertex >= 0 && poll_limit <= 0)) return XPBD_ERR_INVALID;
+    XPBD_CU(c, cudaStreamSynchronize(c->stream));  // no sweep in flight reads the tables
+    const int P = c->pcol_off.back(), ncta = c->cl_shape.ncta;
+    if (c->cl_ver_h.empty()) {
+        c->cl_ver_h.resize(P);
+        XPBD_CU(c, cudaMemcpy(c->cl_ver_h.data(), c->cl.ver, sizeof(int4) * P, cudaMemcpyDeviceToHost));
+    }
+    std::vector<int4> ver = c->cl_ver_h;
+    bool shared = false;
+    if (vertex >= 0) {
+        std::vector<int4> part(2 * (size_t)ncta), vidx(P), meta(P);
+        XPBD_CU(c, cudaMemcpy(part.data(), c->cl.part, sizeof(int4) * part.size(), cudaMemcpyDeviceToHost));
+        XPBD_CU(c, cudaMemcpy(vidx.data(), c->cl.vidx, sizeof(int4) * P, cudaMemcpyDeviceToHost));
+        XPBD_CU(c, cudaMemcpy(meta.data(), c->cl.meta, sizeof(int4) * P, cudaMemcpyDeviceToHost));
+        for (int b = 0; b < ncta; b++) {
+            const int4 pa = part[2 * b], pb = part[2 * b + 1];
+            std::vector<int> verts(pa.z);  // the shared ones
+            XPBD_CU(c, cudaMemcpy(verts.data(), c->cl.verts + pa.x, sizeof(int) * verts.size(), cudaMemcpyDeviceToHost));
+            for (int l = 0; l < pa.z; l++) {
+                if ((verts[l] & 0x7fffffff) != vertex) continue;
+                shared = true;
+                for (int i = pa.w; i < pa.w + pb.x; i++)
+                    for (int k = 0; k < (meta[i].y >> 8); k++)
+                        if ((((&vidx[i].x)[k >> 1] >> (16 * (k & 1))) & 0xffff) == l)
+                            (&ver[i].x)[k >> 1] |= 0xff << (16 * (k & 1));  // pre = 255
+            }
+        }
+        if (!shared) return fail(c, XPBD_ERR_STATE, "vertex %d lies in one block: nothing waits for it", vertex);
+    }
+    XPBD_CU(c, cudaMemcpy((void*)c->cl.ver, ver.data(), sizeof(int4) * P, cudaMemcpyHostToDevice));
+    c->cl_shape.polls = vertex >= 0 ? (unsigned)poll_limit : kClusterPolls;
+    c->graph_dirty = true;  // the poll limit is a launch argument
+    return XPBD_OK;
+}
+
 int xpbd_health(xpbd_ctx* c, int64_t* nonfinite, int64_t* degenerate) {
     if (!c) return XPBD_ERR_INVALID;
     XPBD_CU(c, cudaStreamSynchronize(c->stream));

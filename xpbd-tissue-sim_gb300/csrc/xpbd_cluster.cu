@@ -116,7 +116,7 @@ __device__ __forceinline__ bool cluster_patch(const TetArrays& t, const BlockVer
                                               const int (&due)[kMaxPatchVerts], const int4& meta, const int* __restrict__ slot, const float4* __restrict__ q0,
                                               const float4* __restrict__ q1, const float4* __restrict__ q2,
                                               float2* __restrict__ sl, float4* __restrict__ scratch, int sstride,
-                                              Flags* flags) {
+                                              unsigned polls, Flags* flags) {
     const int ntets = HEX ? kMaxPatchTets : (meta.y & 0xff);
     const int nverts = HEX ? kMaxPatchVerts : (meta.y >> 8);
     const int vw[4] = {vi.x, vi.y, vi.z, vi.w};
@@ -140,7 +140,7 @@ __device__ __forceinline__ bool cluster_patch(const TetArrays& t, const BlockVer
     if (MULTI) {
         // every corner again in one go (the loads overlap), the pending ones taken
         for (unsigned n = 0; pending; n++) {
-            if (n > kClusterPolls) return false;
+            if (n > polls) return false;
             VertWord v[kMaxPatchVerts];
 #pragma unroll
             for (int k = 0; k < kMaxPatchVerts; k++) v[k] = ld_vert(bv.sv + l8[k]);
@@ -380,10 +380,12 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
             if (sh) sw[l] = q.w;
         }
     }
-    bool ok = mbar_wait_bounded(&tbar, 0, kWaitLimit);
+    // without its tables a block neither projects nor touches the multipliers
+    const bool tables = __syncthreads_and(mbar_wait_bounded(&tbar, 0, kWaitLimit)) != 0;
+    bool ok = tables;
     if (first_zero) {
         for (int i = tid; i < ntets; i += nt) slam[i] = make_float2(0.f, 0.f);
-    } else {
+    } else if (tables) {
         for (int i = tid; i < np; i += nt) {
             const int4 m = tm[i];
             const int slot = __ldg(a.slot + p0 + i);
@@ -431,19 +433,26 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     };
     const BlockVerts<MULTI> bv{sv, sw, rem, nb};
     if (MULTI || wid <= producer) {
-        int seq = 0;
+        int seq = 0, staged = nne > 0 ? 1 : 0;  // copies issued (the producer's first lane counts them)
         for (int it = 0; it < iters; it++) {
             for (int pc = 0; pc < passes * s.ncol; pc++) {
                 const int pass = SEPARATE && pc >= s.ncol ? 1 : 0, c = pc - pass * s.ncol;
                 const int4 rg = srg[c];
                 const int n = rg.y;
                 if (wid == producer) {
-                    // the next colour's records into the other buffer, whose readers passed the last barrier
+                    // The next colour's records into the other buffer, whose readers passed the
+                    // last barrier. They waited for the copy before it in that buffer, unless a
+                    // wait of theirs gave up: so it is waited for here too (it has landed), and
+                    // nothing is staged after one that has not.
                     if (!s.resident && n > 0) {
-                        if (lane == 0 && seq + 1 < total) {
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            copy_records(sne[(seq + 1) % nne], rec + ((seq + 1) & 1) * 3 * (size_t)s.rec_cap,
-                                         &bar[(seq + 1) & 1]);
+                        if (lane == 0 && seq + 1 < total && ok) {
+                            if (seq > 0) ok = mbar_wait_bounded(&bar[(seq - 1) & 1], ((seq - 1) >> 1) & 1, kWaitLimit);
+                            if (ok) {
+                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                                copy_records(sne[(seq + 1) % nne], rec + ((seq + 1) & 1) * 3 * (size_t)s.rec_cap,
+                                             &bar[(seq + 1) & 1]);
+                                staged = seq + 2;
+                            }
                         }
                         seq++;
                     }
@@ -487,7 +496,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                         const float4* b0r = buf + (meta.x - rsub);
                         const int* slot = a.slot + p0 + rg.x + q;
 #define XG_PATCH(W, H) ok = cluster_patch<W, H, MULTI>(t, bv, vi, due, meta, slot, b0r, b0r + s.rec_cap, b0r + 2 * s.rec_cap, \
-                                                  slam + meta.x, scratch + tid, 32 * cw, flags)
+                                                  slam + meta.x, scratch + tid, 32 * cw, s.polls, flags)
                         if (SEPARATE) {
                             if (pass == 0) { if (hex) XG_PATCH(0, true); else XG_PATCH(0, false); }
                             else { if (hex) XG_PATCH(1, true); else XG_PATCH(1, false); }
@@ -538,7 +547,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                             }
                             if (MULTI) {
                                 for (unsigned n = 0; pending && ok; n++) {
-                                    if (n > kClusterPolls) ok = false;
+                                    if (n > s.polls) ok = false;
 #pragma unroll
                                     for (int q = 0; q < 3; q++) {
                                         float4 p;
@@ -574,12 +583,17 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                 }
             }
         }
+        // no block leaves with a copy into it in flight (after a wait that gave
+        // up there may be: the last one in each buffer)
+        if (wid == producer && lane == 0)
+            for (int k = staged > 1 ? staged - 2 : 0; k < staged; k++)
+                ok = mbar_wait_bounded(&bar[k & 1], (k >> 1) & 1, kWaitLimit) && ok;
     }
     // a copy or a neighbour's vertex that never came: counted; the work after it
-    // was skipped (the staging copies get a last bounded chance)
+    // was skipped (the tables get a last bounded chance)
     if (!__syncthreads_and(ok) && tid == 0) {
         atomicAdd(&flags->timeouts, 1ull);
-        for (int k = 0; k < 2; k++) mbar_wait_bounded(&bar[k], 0, kWaitLimit);
+        if (!tables) mbar_wait_bounded(&tbar, 0, kWaitLimit);
     }
     if (MULTI) cluster_sync_all();  // the other blocks' last stores are here
     // owners write the vertices back; every block its multipliers
@@ -612,7 +626,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
             io.x[g] = xx;
         }
     }
-    for (int i = tid; i < np; i += nt) {
+    for (int i = tid; tables && i < np; i += nt) {
         const int4 m = tm[i];
         const int slot = __ldg(a.slot + p0 + i);
         for (int k = 0; k < (m.y & 0xff); k++) t.lam[slot + k] = slam[m.x + k];

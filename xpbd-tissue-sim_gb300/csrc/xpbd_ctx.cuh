@@ -142,6 +142,7 @@ struct xpbd_ctx {
     xg::ClusterShape cl_shape{};
     xg::ClusterArrays cl{};
     DevBuf<int4> cl_tab;
+    std::vector<int4> cl_ver_h;  // xpbd_debug_stall_on_chip: the table it changes, as built
     DevBuf<int> cl_ifl, cl_ifo, cl_act_faces, cl_act_off;
     DevBuf<float4> c_bary, c_p, c_n;
     DevBuf<float> c_lam;

@@ -187,7 +187,7 @@ constexpr int kResidentTasks = 10;
 constexpr int kClusterLanes = 128;       // patches of one colour a block projects at once: one warp per scheduler
 constexpr int kClusterThreads = 256;     // most threads of a block
 constexpr int kMaxClusterSize = 16;      // blocks of a cluster (above 8: opt-in)
-constexpr unsigned kClusterPolls = 1u << 20;  // polls of a shared vertex before a wait gives up
+constexpr unsigned kClusterPolls = 1u << 20;  // ClusterShape::polls
 constexpr int kMaxClusterColours = 64;   // patch colours, as build_cluster splits them
 constexpr int kClusterSmemMax = 230400;  // dynamic shared memory of a block (227 KB less the static part)
 struct ClusterArrays {
@@ -216,6 +216,7 @@ struct ClusterShape {
     int max_nv, max_nb, max_p, max_t, max_send;  // largest block: vertices, shared ones, patches, tets, sends
     int rec_cap;                       // tet records of one staging buffer
     int resident;                      // 1: every record stays in shared memory; 0: two buffers, one colour each
+    unsigned polls;                    // of a shared vertex before a wait gives up
     size_t smem;
 };
 // what a one-launch sweep does around its iterations
