@@ -358,6 +358,11 @@ int xpbd_debug_stall_vertex(xpbd_ctx* ctx, int32_t vertex, int32_t poll_limit);
  * 4): the waits for a vertex that two blocks hold run out. XPBD_ERR_STATE where
  * the context has no such sweep, or the vertex lies in one block. */
 int xpbd_debug_stall_on_chip(xpbd_ctx* ctx, int32_t vertex, int32_t poll_limit);
+/* Test hook: how the next substep's sweeps run. route: 0 a launch for each colour
+ * (or Jacobi), 1 one launch with task counters, 2 the versioned sweep, 3 on
+ * chip; on chip also the blocks of an instance's cluster and how many such
+ * clusters the device holds at once (else 0). */
+int xpbd_debug_sweep_route(xpbd_ctx* ctx, int32_t* route, int32_t* cluster_blocks, int32_t* clusters_held);
 /* Colouring in use (coloured Gauss-Seidel). Tets are grouped into patches
  * (runs of up to gs_patch_tets consecutive tets on at most 8 vertices) and the
  * patches are coloured so that patches of one colour share no vertex; each

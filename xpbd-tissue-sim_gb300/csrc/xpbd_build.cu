@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -530,10 +531,12 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
     const std::vector<ClusterChoice> choices =
         part_of.choices(kClusterLanes, kMaxClusterSize, sms, c->prm.self_collisions != 0, separate ? 1.65 : 1.1,
                         separate ? 2.2 : 1.4, other);
+    int too_wide = INT_MAX;  // clusters of this many blocks did not all fit the device
     const int colours = ncol;
     const std::vector<int>& colour_of = ps.colour;
     for (const ClusterChoice& ch : choices) {
         if (ch.us >= other * colours) break;
+        if (ch.n >= too_wide) continue;
         ncol = colours;
         pcol = colour_of;
         part_of.assign(ch.shape, ch.n);
@@ -737,7 +740,16 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
             fl[f] = make_int4(local[slot_in(e[0], home)], local[slot_in(e[1], home)], local[slot_in(e[2], home)],
                               deg[e[0]] | deg[e[1]] << 8 | deg[e[2]] << 16);
         }
-        if (sweep_cluster_fits(s, separate, false) <= 0 || (fok && sweep_cluster_fits(s, separate, true) <= 0)) continue;
+        // In a second wave of clusters a sweep costs twice the estimate, which no
+        // choice below the other route's can afford (20 sweeps of 9 instances of
+        // 22^3 hexes, eleven blocks each: 549 us in two waves, 425 us by the
+        // versioned sweep; 8 of them 282 us).
+        s.held = sweep_cluster_fits(s, separate, false);
+        if (fok) s.held = std::min(s.held, sweep_cluster_fits(s, separate, true));
+        if (s.held < K) {
+            too_wide = std::min(too_wide, csize);
+            continue;
+        }
         if (!fok) fl.clear();
         // one device buffer for the tables
         std::vector<int4> tab;

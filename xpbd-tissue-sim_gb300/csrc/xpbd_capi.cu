@@ -206,6 +206,17 @@ bool use_cluster(const xpbd_ctx* c) {
            (!c->F || c->cluster_contacts || !c->static_seen);
 }
 
+// Whether every iteration and colour of the substep's sweeps is in one
+// cooperative launch (with faces: the versioned sweep, static contacts after
+// each iteration's patches)
+bool use_one_launch(const xpbd_ctx* c) {
+    const xpbd_params& p = c->prm;
+    return p.solver_type != XPBD_SOLVER_JACOBI && !use_cluster(c) && p.constraint_type != XPBD_CONSTRAINT_SEPARATE &&
+           p.residual_policy != XPBD_RESIDUAL_EVERY_ITERATION && c->att_v.empty() &&
+           (!c->F || (p.gs_variant == 4 && c->flow_versioned && c->flow_contacts && !c->self_on && !c->nbodies)) &&
+           (p.gs_variant == 2 || p.gs_variant == 3 || p.gs_variant == 4) && c->ntasks > 0;
+}
+
 // A mesh whose largest colour is at most one warp of patches keeps the inertial
 // move, the copies into and out of the sweep's records and the velocities in
 // their own launches: the number of launches a substep of such a mesh makes is
@@ -247,10 +258,7 @@ int enqueue_update(xpbd_ctx* c, bool write_vel, bool solve_only) {
     const bool jacobi = p.solver_type == XPBD_SOLVER_JACOBI;
     // every iteration and colour in one cooperative launch (with faces: the
     // versioned sweep, static contacts after each iteration's patches)
-    const bool one_launch =
-        !jacobi && !cluster && !separate && !every_iter && c->att_v.empty() &&
-        (!have_faces || (p.gs_variant == 4 && c->flow_versioned && c->flow_contacts && !c->self_on && !c->nbodies)) &&
-        (p.gs_variant == 2 || p.gs_variant == 3 || p.gs_variant == 4) && c->ntasks > 0;
+    const bool one_launch = use_one_launch(c);
     const bool versioned = one_launch && p.gs_variant == 4 && c->flow_versioned;
     // the inertial move is part of the on-chip sweep's launch, or of the
     // versioned sweep's copy into its records, when nothing reads the predicted
@@ -1498,6 +1506,15 @@ int xpbd_debug_stall_vertex(xpbd_ctx* c, int32_t vertex, int32_t poll_limit) {
     c->stalled = vertex >= 0;
     XPBD_CU(c, cudaMemcpy(c->patch_ver.p, ver.data(), sizeof(int4) * ver.size(), cudaMemcpyHostToDevice));
     c->graph_dirty = true;  // the poll limit is a launch argument
+    return XPBD_OK;
+}
+
+int xpbd_debug_sweep_route(xpbd_ctx* c, int32_t* route, int32_t* cluster_blocks, int32_t* clusters_held) {
+    if (!c || !route || !cluster_blocks || !clusters_held) return XPBD_ERR_INVALID;
+    const bool chip = use_cluster(c);
+    *route = chip ? 3 : (!use_one_launch(c) ? 0 : (c->prm.gs_variant == 4 && c->flow_versioned ? 2 : 1));
+    *cluster_blocks = chip ? c->cl_shape.csize : 0;
+    *clusters_held = chip ? c->cl_shape.held : 0;
     return XPBD_OK;
 }
 

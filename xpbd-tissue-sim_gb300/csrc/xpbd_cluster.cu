@@ -672,8 +672,9 @@ void cluster_config(const Launch& L, const ClusterShape& s, cudaLaunchConfig_t& 
         }                                                                                 \
     } while (0)
 
-// Prepares the kernel for this shape; returns how many clusters of it fit the
-// device at once (0: it cannot run).
+// Prepares the kernel for this shape; returns how many clusters of it the
+// device holds at once (0: it cannot run). The blocks of a cluster share a GPC:
+// a GB300 holds 8 clusters of eleven blocks, not 13.
 int sweep_cluster_fits(const ClusterShape& s, bool separate, bool contacts) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
@@ -690,11 +691,16 @@ int sweep_cluster_fits(const ClusterShape& s, bool separate, bool contacts) {
     } while (0)
     XG_CLUSTER_EACH(XG_DO);
 #undef XG_DO
+    int dev = 0, sms = 1;
+    if (e == cudaSuccess && s.csize == 1) {
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    return n;
+    return n * sms;
 }
 
 cudaError_t launch_sweep_cluster(const Launch& L, const ClusterArrays& a, const ClusterShape& s, const TetArrays& t,

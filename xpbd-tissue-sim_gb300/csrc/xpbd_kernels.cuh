@@ -216,6 +216,7 @@ struct ClusterShape {
     int max_nv, max_nb, max_p, max_t, max_send;  // largest block: vertices, shared ones, patches, tets, sends
     int rec_cap;                       // tet records of one staging buffer
     int resident;                      // 1: every record stays in shared memory; 0: two buffers, one colour each
+    int held;                          // clusters the device holds at once
     unsigned polls;                    // of a shared vertex before a wait gives up
     size_t smem;
 };
@@ -380,7 +381,7 @@ void launch_versions_out(const Launch& s, float4* x, const VerRec* xv, const int
 cudaError_t launch_sweep_cluster(const Launch& s, const ClusterArrays& a, const ClusterShape& sh, const TetArrays& t,
                                  const ClusterIo& io, int iters, bool first_zero, bool separate, bool contacts,
                                  const ContactArrays& ca, Flags* flags);
-// clusters of this shape that fit the device at once (0: it cannot run)
+// clusters of this shape that the device holds at once (0: it cannot run)
 int sweep_cluster_fits(const ClusterShape& sh, bool separate, bool contacts);
 // After a detection (the per-instance active lists built): the sweep's
 // contact tables. vface_off/vface/fcol/vdegp are static: per vertex its

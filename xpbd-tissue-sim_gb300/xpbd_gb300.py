@@ -139,6 +139,7 @@ def load(path: str | None = None):
         "xpbd_health": ([P, P, P], C.c_int),
         "xpbd_debug_stall_vertex": ([P, I32, I32], C.c_int),
         "xpbd_debug_stall_on_chip": ([P, I32, I32], C.c_int),
+        "xpbd_debug_sweep_route": ([P, P, P, P], C.c_int),
         "xpbd_num_colours": ([P, P, P], C.c_int),
         "xpbd_get_tet_colours": ([P, P], C.c_int),
         "xpbd_get_sweep_order": ([P, P], C.c_int),
@@ -504,6 +505,13 @@ class XPBDSolver:
         """Test hook: the same for the on-chip sweep's waits on a vertex that two
         blocks hold."""
         self._ck(self.L.xpbd_debug_stall_on_chip(self.h, int(vertex), int(poll_limit)))
+
+    def debug_sweep_route(self):
+        """Test hook: ("launches" | "counters" | "versioned" | "chip", blocks of a
+        cluster, clusters the device holds at once) of the next substep's sweeps."""
+        r = [C.c_int32() for _ in range(3)]
+        self._ck(self.L.xpbd_debug_sweep_route(self.h, *(C.byref(v) for v in r)))
+        return ("launches", "counters", "versioned", "chip")[r[0].value], r[1].value, r[2].value
 
     def colours(self):
         nt, nf = C.c_int32(), C.c_int32()
