@@ -4,6 +4,7 @@ library's index checks on."""
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -149,3 +150,64 @@ def test_no_vertex_lies_in_more_than_two_blocks(planner, K, dims):
     assert all(int(most) <= 2 for _, _, _, most in rows), rows
     if K == 1 and dims == (10, 100, 10):  # the beam keeps its slabs
         assert rows[0][:2] == ["10", "1"]
+
+
+GROUPS = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "xpbd_partition.hpp"
+// stdin: warps, K, ncol, counts by instance; out: the groups' first instances and K
+int main() {
+    long long warps;
+    int K, ncol;
+    if (std::scanf("%lld %d %d", &warps, &K, &ncol) != 3) return 2;
+    std::vector<std::vector<int>> n(K, std::vector<int>(ncol));
+    for (auto& r : n)
+        for (int& v : r)
+            if (std::scanf("%d", &v) != 1) return 2;
+    for (int g : xg::host::task_groups(n, 32, warps)) std::printf("%d ", g);
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def grouper(tmp_path_factory):
+    d = tmp_path_factory.mktemp("groups")
+    src, exe = str(d / "g.cpp"), str(d / "g")
+    open(src, "w").write(GROUPS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-D_GLIBCXX_ASSERTIONS", "-I",
+                    os.path.join(ROOT, "xpbd-tissue-sim_gb300", "csrc"), src, "-o", exe], check=True)
+    return exe
+
+
+def _rounds(counts, first, warps):
+    tasks = sum(max(1, -(-int(counts[a:b].sum(0).max()) // 32)) for a, b in zip(first[:-1], first[1:]))
+    return -(-tasks // warps)
+
+
+@pytest.mark.parametrize("name,warps", [("tiny", 1216), ("tiny", 1), ("uneven", 1216), ("just_over", 1216),
+                                        ("mixed", 1216), ("one", 1216), ("odd_colours", 100)])
+def test_small_instances_share_tasks_only_where_that_saves_rounds(grouper, name, warps):
+    """Tasks of the dataflow sweeps: never more rounds of the warps than equal
+    shares of the union of all instances take; every instance by itself where
+    that costs no round more."""
+    rng = np.random.default_rng(0)
+    counts = {"tiny": np.tile([6, 4, 4, 4, 6, 4, 4, 2], (5000, 1)),       # 40 hexes each
+              "uneven": rng.integers(40, 1800, (96, 1)) + rng.integers(0, 9, (96, 8)),
+              "just_over": np.tile([40, 36, 36, 32, 40, 36, 36, 32], (700, 1)),
+              "mixed": np.concatenate([np.full((2000, 8), 3), np.full((3, 8), 9000)]),
+              "one": np.full((1, 8), 32768),
+              "odd_colours": rng.integers(0, 50, (640, 13))}[name]
+    text = f"{warps} {len(counts)} {counts.shape[1]} " + " ".join(map(str, counts.ravel()))
+    r = subprocess.run([grouper], input=text, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    first = [int(v) for v in r.stdout.split()]
+    assert first[0] == 0 and first[-1] == len(counts) and all(b > a for a, b in zip(first, first[1:]))
+    got, union = _rounds(counts, first, warps), _rounds(counts, [0, len(counts)], warps)
+    alone = _rounds(counts, list(range(len(counts) + 1)), warps)
+    assert got <= min(union, alone)
+    if alone == union:
+        assert len(first) == len(counts) + 1
+    if name in ("tiny", "just_over") and warps > 1:
+        assert got < alone

@@ -45,3 +45,32 @@ def test_on_chip_clusters_fit_the_device_and_agree_with_the_versioned_sweep(lib,
         s.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_small_instances_that_share_tasks_equal_each_alone(lib):
+    """1,500 instances of 12 hexes: more than the device has warps for, so a task
+    of the versioned sweep holds patches of several of them. An instance's
+    states equal those of a context of its own bit for bit."""
+    X, tets, _ = G.grid_mesh(2, 3, 2, 0.01)
+    K = 1500
+    rng = np.random.default_rng(2)
+    E = np.exp(rng.uniform(np.log(1e3), np.log(1e4), (K, len(tets))))
+    x = np.stack([X + 5e-4 * rng.uniform(-1, 1, X.shape) for _ in range(K)])
+
+    def run(ks):
+        s = G.XPBDSolver(instances=[(X, tets, None, E[k], 0.45, 1000.0) for k in ks], num_iters=5, collision_rate=0.0)
+        s.fix_vertices(np.tile(X[:, 2] == 0, len(ks)))
+        s.set_positions(x[ks].reshape(-1, 3))
+        if len(ks) > 1:
+            assert s.debug_sweep_route()[0] == "versioned"
+        s.step(3)
+        s.synchronize()
+        out = s.positions().reshape(len(ks), -1, 3), s.lambdas().reshape(len(ks), len(tets), 2)
+        s.close()
+        return out
+
+    P, lam = run(list(range(K)))
+    for k in (0, 1, 37, 700, 1499):
+        p, m = run([k])
+        np.testing.assert_array_equal(P[k], p[0])
+        np.testing.assert_array_equal(lam[k], m[0])

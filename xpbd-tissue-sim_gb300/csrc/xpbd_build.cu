@@ -150,36 +150,70 @@ void release(xpbd_ctx* c) {
 // vertex with it, flagged when theirs is the higher colour.
 int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector<int4>& pverts) {
     const int P = (int)pmeta.size(), V = c->V;
+    auto pv = [&](int q, int k) {
+        const int4& a = pverts[2 * (size_t)q + (k >> 2)];
+        const int kk = k & 3;
+        return kk == 0 ? a.x : (kk == 1 ? a.y : (kk == 2 ? a.z : a.w));
+    };
+    std::vector<int> voff(V + 1, 0);
+    for (int q = 0; q < P; q++)
+        for (int k = 0; k < (pmeta[q].y >> 8); k++) voff[pv(q, k) + 1]++;
+    // the versioned sweep orders itself by vertex versions: only where a vertex
+    // has more patches than its fields hold (below) does it need the lists
+    const bool lists = c->prm.gs_variant != 4 || *std::max_element(voff.begin(), voff.end()) > 255;
+    const bool staged = c->prm.gs_variant == 3;
+    // variant 4 falls back to variant 2 (below) where it needs the lists
+    const bool with_faces = c->F > 0;  // variant 4 may then run the contacts inside the sweep
+    int per_sm = lists ? sweep_dataflow_blocks_per_sm(staged, c->prm.gs_min_blocks) : 1 << 20;
+    if (c->prm.gs_variant == 4) {
+        per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, false));
+        if (with_faces) per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, true));
+    }
+    int dev = 0, sms = 0;
+    XPBD_CU(c, cudaGetDevice(&dev));
+    XPBD_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (per_sm <= 0 || sms <= 0) return fail(c, XPBD_ERR_CUDA, "dataflow sweep: no co-resident blocks");
+    const int warps = per_sm * sms * ((staged ? kPatchBlock : kFlowBlock) / 32);  // co-resident
     std::vector<int4> tasks;
     std::vector<int> tcol, task_of(P);
-    // Within an instance, every colour in as many tasks as the largest one needs,
-    // each with an equal share of its patches (both follow the mesh order): the
-    // k-th tasks of the colours then cover the same part of the mesh, also where
-    // the colours differ in size, and a warp mostly waits for its own earlier
-    // tasks. (With runs of 32 the k-th tasks drift apart: per colour of a sweep
-    // 3.95 against 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47 x 49
-    // x 45, the same for 48 x 48 x 48; shares of the union of 96
-    // uneven instances instead of each one's: 4.17 against 3.99 ms a pass.)
+    // Within a group of instances, every colour in as many tasks as the largest
+    // one needs, each with an equal share of its patches (both follow the mesh
+    // order): the k-th tasks of the colours then cover the same part of the mesh,
+    // also where the colours differ in size, and a warp mostly waits for its own
+    // earlier tasks. (With runs of 32 the k-th tasks drift apart: per colour of a
+    // sweep 3.95 against 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47
+    // x 49 x 45, the same for 48 x 48 x 48; shares of the union of 96 uneven
+    // instances instead of each one's: 4.17 against 3.99 ms a pass.) Small
+    // instances share tasks where one each would take the warps more rounds
+    // (task_groups): a substep of 20 sweeps of 5,000 instances of 40 hexes, five
+    // lanes a task in five rounds, took 1,790 us, shares of the union 426.
     const int K = c->n_inst, ncol = c->n_tet_colours;
     std::vector<int> first((size_t)ncol * (K + 1));  // [colour][instance] first patch
-    std::vector<int> per_colour(K, 1);
+    std::vector<std::vector<int>> count(K, std::vector<int>(ncol));
     for (int col = 0; col < ncol; col++) {
         int q = c->pcol_off[col];
         for (int k = 0; k <= K; k++) {
             while (k > 0 && q < c->pcol_off[col + 1] && c->tet_of_slot[pmeta[q].x] < c->toff[k]) q++;
             first[(size_t)col * (K + 1) + k] = q;
-            if (k > 0) {
-                const int n = q - first[(size_t)col * (K + 1) + k - 1];
-                per_colour[k - 1] = std::max(per_colour[k - 1], (n + kTaskPatches - 1) / kTaskPatches);
-            }
+            if (k > 0) count[k - 1][col] = q - first[(size_t)col * (K + 1) + k - 1];
         }
     }
+    const std::vector<int> group = task_groups(count, kTaskPatches, warps);
+    const int G = (int)group.size() - 1;
+    auto patches = [&](int col, int g) {  // of a group and colour: first, number
+        const int* f = &first[(size_t)col * (K + 1)];
+        return std::make_pair((long long)f[group[g]], (long long)f[group[g + 1]] - f[group[g]]);
+    };
+    std::vector<int> per_colour(G, 1);
     for (int col = 0; col < ncol; col++)
-        for (int k = 0; k < K; k++) {
-            const long long q0 = first[(size_t)col * (K + 1) + k], count = first[(size_t)col * (K + 1) + k + 1] - q0;
-            for (int i = 0; i < per_colour[k]; i++) {
-                const int q = (int)(q0 + count * i / per_colour[k]);
-                const int n = (int)(q0 + count * (i + 1) / per_colour[k]) - q;
+        for (int g = 0; g < G; g++)
+            per_colour[g] = std::max(per_colour[g], (int)((patches(col, g).second + kTaskPatches - 1) / kTaskPatches));
+    for (int col = 0; col < ncol; col++)
+        for (int g = 0; g < G; g++) {
+            const auto [q0, share] = patches(col, g);
+            for (int i = 0; i < per_colour[g]; i++) {
+                const int q = (int)(q0 + share * i / per_colour[g]);
+                const int n = (int)(q0 + share * (i + 1) / per_colour[g]) - q;
                 int slots = 0;
                 for (int j = 0; j < n; j++) {
                     task_of[q + j] = (int)tasks.size();
@@ -193,18 +227,7 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
             }
         }
     const int NT = (int)tasks.size();
-    auto pv = [&](int q, int k) {
-        const int4& a = pverts[2 * (size_t)q + (k >> 2)];
-        const int kk = k & 3;
-        return kk == 0 ? a.x : (kk == 1 ? a.y : (kk == 2 ? a.z : a.w));
-    };
     // vertex -> tasks (CSR, deduplicated)
-    std::vector<int> voff(V + 1, 0);
-    for (int q = 0; q < P; q++)
-        for (int k = 0; k < (pmeta[q].y >> 8); k++) voff[pv(q, k) + 1]++;
-    // the versioned sweep orders itself by vertex versions: only where a vertex
-    // has more patches than its fields hold (below) does it need the lists
-    const bool lists = c->prm.gs_variant != 4 || *std::max_element(voff.begin(), voff.end()) > 255;
     for (int v = 0; v < V; v++) voff[v + 1] += voff[v];
     std::vector<int> vt(lists ? voff[V] : 0), fill(voff.begin(), voff.end() - 1);
     for (int q = 0; q < P && lists; q++)
@@ -228,18 +251,6 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
         }
         doff[j + 1] = (int)dep.size();
     }
-    const bool staged = c->prm.gs_variant == 3;
-    // variant 4 falls back to variant 2 (below) where it needs the lists
-    const bool with_faces = c->F > 0;  // variant 4 may then run the contacts inside the sweep
-    int per_sm = lists ? sweep_dataflow_blocks_per_sm(staged, c->prm.gs_min_blocks) : 1 << 20;
-    if (c->prm.gs_variant == 4) {
-        per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, false));
-        if (with_faces) per_sm = std::min(per_sm, sweep_versioned_blocks_per_sm(c->prm.gs_min_blocks, 0, true));
-    }
-    int dev = 0, sms = 0;
-    XPBD_CU(c, cudaGetDevice(&dev));
-    XPBD_CU(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (per_sm <= 0 || sms <= 0) return fail(c, XPBD_ERR_CUDA, "dataflow sweep: no co-resident blocks");
     c->flow_grid = per_sm * sms;
     if (!staged) {
         // no more warps than the largest colour has tasks

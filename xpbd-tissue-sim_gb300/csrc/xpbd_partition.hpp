@@ -176,5 +176,54 @@ private:
     }
 };
 
+// Which consecutive instances share the tasks of the dataflow sweeps. A colour of
+// a group goes into ceil(m / lanes) tasks, m the patches of its largest colour;
+// `warps` warps take the tasks in rounds. count: per instance the patches of each
+// colour. Returns the groups' first instances and, last, the number of
+// instances: every instance by itself while that costs no round more than fuller
+// tasks would, else the smallest groups with the fewest rounds.
+inline std::vector<int> task_groups(const std::vector<std::vector<int>>& count, int lanes, long long warps) {
+    const int K = (int)count.size();
+    auto groups = [&](long long cap, long long& tasks) {  // of at most cap patches of one colour, or one instance
+        std::vector<int> first;
+        std::vector<long long> sum, with;
+        long long m = 0;
+        tasks = 0;
+        auto close = [&] {
+            if (!first.empty()) tasks += std::max(1LL, (m + lanes - 1) / lanes);
+        };
+        for (int k = 0; k < K; k++) {
+            with = sum;
+            long long w = 0;
+            for (size_t c = 0; c < count[k].size() && !first.empty(); c++) w = std::max(w, with[c] += count[k][c]);
+            if (first.empty() || w > cap) {
+                close();
+                first.push_back(k);
+                with.assign(count[k].begin(), count[k].end());
+                w = with.empty() ? 0 : *std::max_element(with.begin(), with.end());
+            }
+            sum.swap(with);
+            m = w;
+        }
+        close();
+        first.push_back(K);
+        return first;
+    };
+    long long all = 0, tasks = 0;
+    for (const auto& c : count)
+        for (int n : c) all += n;
+    std::vector<int> best = groups(0, tasks);
+    long long rounds = (tasks + warps - 1) / warps;
+    for (long long cap = lanes; rounds > 1; cap *= 2) {
+        const std::vector<int> g = groups(cap, tasks);
+        if ((tasks + warps - 1) / warps < rounds) {
+            rounds = (tasks + warps - 1) / warps;
+            best = g;
+        }
+        if (cap > all) break;
+    }
+    return best;
+}
+
 }  // namespace host
 }  // namespace xg
