@@ -265,7 +265,7 @@ struct SelfArrays {
     int* plan;              // [n_surf] contacts, round by round
     int4* plan_ids;         // [n_surf] their vertices
     int* round_off;         // [n_surf + 2] the rounds' ranges
-    int* n_rounds;          // [1] -1: too many contacts, in detection order instead
+    int* n_rounds;          // [1] -1: no plan, one by one in detection order
     int* owner;             // [V] scratch
     int V;
 };

@@ -421,12 +421,11 @@ __device__ float self_contact_eval(const float* q, const float* p1, const float*
 }
 
 // ConstraintProjector::project (ConstraintProjector.hpp:111-172) of self
-// contact j on the vertices ids (surface vertex, face): skipped when C > 0;
+// contact j on the vertices xs (surface vertex, face): skipped when C > 0;
 // alpha~ = 1e-8/dt^2 (or /dt)
-__device__ bool self_update(const SelfArrays& a, int j, const int4& ids, const float4* x, bool first, float at,
-                            float4 xs[4], float d[4][3], Flags* flags) {
+__device__ bool self_update(const SelfArrays& a, int j, bool first, float at, const float4 xs[4], float d[4][3],
+                            Flags* flags) {
     float lam = first ? 0.f : a.lam[j];
-    xs[0] = x[ids.x]; xs[1] = x[ids.y]; xs[2] = x[ids.z]; xs[3] = x[ids.w];
     float p[4][3];
     for (int i = 0; i < 4; i++) {
         p[i][0] = xs[i].x; p[i][1] = xs[i].y; p[i][2] = xs[i].z;
@@ -466,14 +465,21 @@ __device__ __forceinline__ int4 self_ids(const SelfArrays& a, int j, const int4*
 // share no vertex, and of two on a common vertex the earlier one is in the
 // earlier round. One block; the bids lie in shared memory, by each vertex's
 // lowest (contact, corner) number, or beyond kPlanShared contacts in owner[].
-// owner is all 0x7f bytes before and after.
+// owner is all 0x7f bytes before.
+// A vertex of many contacts takes a round for each of them, in which all that are
+// left bid again: 10,201 contacts, 9,460 of them on one face, took 226 ms to plan
+// and lost by it (four sweeps 41.0 ms in rounds, 34.0 one by one). So there is no
+// plan (n_rounds -1, the projection walks the list) where a vertex has more than
+// plan_rounds(n) contacts or the rounds get to be more. Two cubes pressed
+// together take about 2 sqrt(n).
 constexpr int kPlanThreads = 1024, kPlanShared = 4096, kPlanMost = 32 * kPlanThreads;
 constexpr int kNoOwner = 0x7f7f7f7f;
+__host__ __device__ constexpr int plan_rounds(int n) { return n < 256 ? 64 : (n < 2048 ? n / 4 : 512); }
 __global__ void __launch_bounds__(kPlanThreads) k_self_plan(SelfArrays a, const int4* __restrict__ faces) {
     extern __shared__ int bids[];  // [4 kPlanShared] bids, [4 kPlanShared] the vertices' numbers
-    __shared__ int placed, left;
+    __shared__ int placed, left, most;
     pdl_wait_then_release();
-    const int n = *a.n_hits, tid = threadIdx.x;
+    const int n = *a.n_hits, tid = threadIdx.x, limit = plan_rounds(n);
     if (n > kPlanMost) {  // more than a thread's 32 bits: the projection walks them one by one
         if (tid == 0) *a.n_rounds = -1;
         return;
@@ -481,7 +487,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_self_plan(SelfArrays a, const 
     const bool small = n <= kPlanShared;
     volatile int* const owner = a.owner;
     unsigned mine = 0;  // contacts tid + 1024 b that are left
-    if (tid == 0) placed = 0;
+    if (tid == 0) placed = most = 0;
     for (int b = 0; tid + kPlanThreads * b < n; b++) {
         const int j = tid + kPlanThreads * b;
         const int4 id = self_ids(a, j, faces);
@@ -508,26 +514,44 @@ __global__ void __launch_bounds__(kPlanThreads) k_self_plan(SelfArrays a, const 
         }
         __syncthreads();
     }
+    volatile int* const own = small ? bids : a.owner;
+    auto each = [&](unsigned set, auto&& f) {
+        for (unsigned m = set; m; m &= m - 1) {
+            const int b = __ffs((int)m) - 1, j = tid + kPlanThreads * b;
+            int at[4];
+            if (small) {
+                for (int k = 0; k < 4; k++) at[k] = bids[4 * kPlanShared + 4 * j + k];
+            } else {
+                const int4 id = self_ids(a, j, faces);
+                at[0] = id.x; at[1] = id.y; at[2] = id.z; at[3] = id.w;
+            }
+            f(b, j, at);
+        }
+    };
+    // the contacts of the vertex that has most, counted down from kNoOwner
+    each(mine, [&](int, int, const int* at) {
+        for (int k = 0; k < 4; k++) atomicSub((int*)own + at[k], 1);
+    });
+    __syncthreads();
+    each(mine, [&](int, int, const int* at) {
+        for (int k = 0; k < 4; k++)
+            if (kNoOwner - own[at[k]] > limit) most = limit + 1;
+    });
+    __syncthreads();
+    if (most > limit) {
+        if (tid == 0) *a.n_rounds = -1;
+        return;
+    }
+    each(mine, [&](int, int, const int* at) {
+        for (int k = 0; k < 4; k++) own[at[k]] = kNoOwner;
+    });
+    __syncthreads();
     int round = 0;
     for (;;) {
         if (tid == 0) {
             a.round_off[round] = placed;
             left = 0;
         }
-        auto each = [&](unsigned set, auto&& f) {
-            for (unsigned m = set; m; m &= m - 1) {
-                const int b = __ffs((int)m) - 1, j = tid + kPlanThreads * b;
-                int at[4];
-                if (small) {
-                    for (int k = 0; k < 4; k++) at[k] = bids[4 * kPlanShared + 4 * j + k];
-                } else {
-                    const int4 id = self_ids(a, j, faces);
-                    at[0] = id.x; at[1] = id.y; at[2] = id.z; at[3] = id.w;
-                }
-                f(b, j, at);
-            }
-        };
-        volatile int* const own = small ? bids : a.owner;
         each(mine, [&](int, int j, const int* at) {
             for (int k = 0; k < 4; k++) atomicMin((int*)own + at[k], j);
         });
@@ -547,25 +571,25 @@ __global__ void __launch_bounds__(kPlanThreads) k_self_plan(SelfArrays a, const 
         if (mine) left = 1;
         __syncthreads();
         round++;
-        if (!left) break;
+        if (!left || round == limit) break;
         __syncthreads();
     }
     if (tid == 0) {
         a.round_off[round] = placed;
-        *a.n_rounds = round;
+        *a.n_rounds = left ? -1 : round;
     }
 }
 
 // Gauss-Seidel: the contacts as in detection (vertex) order, by the rounds of
 // k_self_plan, one block. (One thread walking the list took 264 us for two
 // 12^3 cubes in contact, four dependent loads and 0.4 us of arithmetic a
-// contact; the rounds 48 us.)
+// contact; the rounds 48 us.) Without a plan one thread walks it.
 constexpr int kSelfGsThreads = 128;
 __device__ __forceinline__ void self_contact_gs(const SelfArrays& a, int j, const int4& ids, float4* __restrict__ x,
                                                 bool first, float at, Flags* flags) {
-    float4 xs[4];
+    const float4 xs[4] = {x[ids.x], x[ids.y], x[ids.z], x[ids.w]};
     float d[4][3];
-    if (!self_update(a, j, ids, x, first, at, xs, d, flags)) return;
+    if (!self_update(a, j, first, at, xs, d, flags)) return;
     const int v[4] = {ids.x, ids.y, ids.z, ids.w};
     if (v[0] != v[1] && v[0] != v[2] && v[0] != v[3] && v[1] != v[2] && v[1] != v[3] && v[2] != v[3]) {
         for (int i = 0; i < 4; i++)
@@ -578,18 +602,52 @@ __device__ __forceinline__ void self_contact_gs(const SelfArrays& a, int j, cons
     }
 }
 
+// Without a plan: one by one, one thread. Such lists have many contacts on one
+// face, whose vertices stay in registers from one contact to the next; the next
+// one's surface vertex is on its way meanwhile (a face or vertex that this
+// contact moves is read after it). 10,201 contacts: 0.83 us each, 0.86 with every
+// vertex read again.
+__device__ void walk_contacts(const SelfArrays& a, const int4* __restrict__ faces, float4* __restrict__ x, bool first,
+                              float at, Flags* flags) {
+    const int n = *a.n_hits;
+    const int4 none = make_int4(-1, -1, -1, -1);
+    int4 ids = n > 0 ? self_ids(a, 0, faces) : none;
+    float4 xs[4] = {};
+    if (ids.x >= 0) { xs[0] = x[ids.x]; xs[1] = x[ids.y]; xs[2] = x[ids.z]; xs[3] = x[ids.w]; }
+    for (int j = 0; j < n; j++) {
+        const int4 next = j + 1 < n ? self_ids(a, j + 1, faces) : none;
+        float4 nx = xs[0];
+        if (next.x >= 0) nx = x[next.x];
+        bool kept = ids.x >= 0;  // xs holds the face's current positions
+        float d[4][3];
+        if (ids.x >= 0 && self_update(a, j, first, at, xs, d, flags)) {
+            const int v[4] = {ids.x, ids.y, ids.z, ids.w};
+            kept = v[0] != v[1] && v[0] != v[2] && v[0] != v[3] && v[1] != v[2] && v[1] != v[3] && v[2] != v[3];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 c = kept ? xs[i] : x[v[i]];  // a vertex may repeat: add to the current value
+                xs[i] = make_float4(c.x + d[i][0], c.y + d[i][1], c.z + d[i][2], c.w);
+                x[v[i]] = xs[i];
+            }
+        }
+        if (next.x >= 0) {
+            if (!(kept && next.y == ids.y && next.z == ids.z && next.w == ids.w)) {
+                xs[1] = x[next.y]; xs[2] = x[next.z]; xs[3] = x[next.w];
+            }
+            const bool moved = next.x == ids.x || next.x == ids.y || next.x == ids.z || next.x == ids.w;
+            xs[0] = moved ? x[next.x] : nx;
+        }
+        ids = next;
+    }
+}
+
 __global__ void __launch_bounds__(kSelfGsThreads) k_self_contacts_gs(SelfArrays a, const int4* __restrict__ faces,
                                                                      float4* __restrict__ x, bool first, float at,
                                                                      Flags* flags) {
     pdl_wait_then_release();
     const int rounds = *a.n_rounds;
     if (rounds < 0) {
-        if (threadIdx.x != 0) return;
-        const int n = *a.n_hits;
-        for (int j = 0; j < n; j++) {
-            const int4 ids = self_ids(a, j, faces);
-            if (ids.x >= 0) self_contact_gs(a, j, ids, x, first, at, flags);
-        }
+        if (threadIdx.x == 0) walk_contacts(a, faces, x, first, at, flags);
         return;
     }
     // a round's first contacts are loaded while the one before runs
@@ -627,9 +685,10 @@ __global__ void k_self_contacts_jacobi(SelfArrays a, const int4* __restrict__ fa
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= *a.n_hits) return;
     const int4 ids = self_ids(a, j, faces);
-    float4 xs[4];
+    if (ids.x < 0) return;
+    const float4 xs[4] = {x[ids.x], x[ids.y], x[ids.z], x[ids.w]};
     float d[4][3];
-    if (ids.x < 0 || !self_update(a, j, ids, x, first, at, xs, d, flags)) return;
+    if (!self_update(a, j, first, at, xs, d, flags)) return;
     const int v[4] = {ids.x, ids.y, ids.z, ids.w};
     for (int i = 0; i < 4; i++) add_vec4(dx + v[i], d[i][0], d[i][1], d[i][2]);
 }
