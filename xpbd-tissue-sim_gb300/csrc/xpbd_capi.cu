@@ -796,18 +796,18 @@ extern "C" {
 
 int xpbd_set_positions(xpbd_ctx* c, const double* x) {
     if (!c || !x) return XPBD_ERR_INVALID;
-    if (c->host_direct) return host_direct_in(c, c->x.p, x, true);
+    if (c->direct(x)) return host_direct_in(c, c->x.p, x, true);
     return stage_positions_to_device(c, x, nullptr);
 }
 
 int xpbd_set_positions_f32(xpbd_ctx* c, const float* x) {
     if (!c || !x) return XPBD_ERR_INVALID;
-    if (c->host_direct) return host_direct_in(c, c->x.p, x, true);
+    if (c->direct(x)) return host_direct_in(c, c->x.p, x, true);
     return stage_positions_to_device(c, nullptr, x);
 }
 
 static int get_xyz(xpbd_ctx* c, const float4* src, double* out) {
-    if (c->host_direct) return host_direct_out(c, out, src);
+    if (c->direct(out)) return host_direct_out(c, out, src);
     int st = fetch(c, src);
     if (st) return st;
     for (int i = 0; i < c->V; i++) {
@@ -825,7 +825,7 @@ int xpbd_get_positions(xpbd_ctx* c, double* x) {
 
 int xpbd_get_positions_f32(xpbd_ctx* c, float* x) {
     if (!c || !x) return XPBD_ERR_INVALID;
-    if (c->host_direct) return host_direct_out(c, x, c->x.p);
+    if (c->direct(x)) return host_direct_out(c, x, c->x.p);
     int st = fetch(c, c->x.p);
     if (st) return st;
     for (int i = 0; i < c->V; i++) {
@@ -843,7 +843,7 @@ int xpbd_get_prev_positions(xpbd_ctx* c, double* x) {
 
 int xpbd_set_velocities(xpbd_ctx* c, const double* v) {
     if (!c || !v) return XPBD_ERR_INVALID;
-    if (c->host_direct) return host_direct_in(c, c->vel.p, v, false);
+    if (c->direct(v)) return host_direct_in(c, c->vel.p, v, false);
     for (int i = 0; i < c->V; i++)
         c->h_stage[i] = make_float4((float)v[3 * i], (float)v[3 * i + 1], (float)v[3 * i + 2], 0.f);
     XPBD_CU(c, cudaMemcpyAsync(c->vel.p, c->h_stage, sizeof(float4) * c->V, cudaMemcpyHostToDevice, c->stream));

@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <string>
 #include <vector>
@@ -198,6 +199,10 @@ struct xpbd_ctx {
     // the device addresses pageable host memory coherently (Grace-Blackwell):
     // positions cross the boundary by kernels on the caller's own arrays
     bool host_direct = false;
+    // whether the device reads or writes this host array itself: an array that is
+    // not aligned to its type is copied by the host
+    template <typename T>
+    bool direct(const T* h) const { return host_direct && reinterpret_cast<uintptr_t>(h) % alignof(T) == 0; }
     double* h_rows = nullptr;
     int h_rows_cap = 0;
     int last_rows = 0;

@@ -153,7 +153,7 @@ struct RowBuffers {
 // the caller's FP32 rows (n x 16) as BF16, and its targets (n x 2, or null):
 // read by the device itself where it addresses pageable host memory
 int upload_rows(xpbd_ctx* c, const float* X, const float* Y, int64_t n, const RowBuffers& d) {
-    if (c->host_direct) {
+    if (c->direct(X) && c->direct(Y)) {
         launch_rows_from_host(c->stream, d.X, X, Y ? d.Y : nullptr, Y, n);
         return cuda_check(c, cudaGetLastError(), "rows from host");
     }
