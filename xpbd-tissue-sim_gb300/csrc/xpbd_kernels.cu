@@ -977,7 +977,8 @@ __global__ void __launch_bounds__(kPatchBlock, 6) k_sweep_dataflow_staged(TetArr
     for (int it = 0; it < iters; it++) {
         for (int j = gw; j < ta.ntasks; j += nw) {
             const int4 tk = __ldg(ta.task + j);
-            if (lane == 0) {
+            const bool copy = tk.w > 0;  // a colour's share may be empty: nothing to copy, no phase
+            if (copy && lane == 0) {
                 // the previous task's reads of sq are done (syncwarp below)
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 const unsigned bytes = (unsigned)tk.w * 16u;
@@ -1025,8 +1026,9 @@ __global__ void __launch_bounds__(kPatchBlock, 6) k_sweep_dataflow_staged(TetArr
                     if (k < nverts) sv[k][tid] = __ldcg(x + vid[k]);
             }
             // the copies land (or not) whatever happened above
-            const bool staged = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[wib], phase, kWaitLimit)) != 0;
-            phase ^= 1u;
+            const bool staged =
+                __all_sync(0xffffffffu, !copy || mbar_wait_bounded(&bar[wib], phase, kWaitLimit)) != 0;
+            if (copy) phase ^= 1u;
             if (!ok || !staged) {
                 if (lane == 0) {
                     atomicExch(ta.abort_flag, 1u);
