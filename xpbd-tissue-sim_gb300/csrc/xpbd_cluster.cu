@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     __shared__ int ssoff[kMaxClusterColours + 1];        // MULTI: its vertices to send per colour
     __shared__ int soff[kMaxFlowFaceColours + 1];        // its active faces per face colour
     __shared__ unsigned long long s_faces;               // face colours active in this block
+    __shared__ int s_stop;                               // a wait for staged records ran out
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
     constexpr int cw = kClusterLanes / 32, producer = cw;  // projecting warps, the record stager
     // the vertices come first: at the same place in every block
@@ -302,6 +303,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     if (MULTI)
         for (int c = tid; c <= s.ncol; c += nt) ssoff[c] = __ldg(a.send_off + (size_t)blockIdx.x * (s.ncol + 1) + c);
     if (tid == 0) {
+        s_stop = 0;
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
         mbar_init(&tbar, 1);
@@ -380,8 +382,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
             if (sh) sw[l] = q.w;
         }
     }
-    // without its tables a block neither projects nor touches the multipliers
-    const bool tables = __syncthreads_and(mbar_wait_bounded(&tbar, 0, kWaitLimit)) != 0;
+    // without its tables a thread neither projects nor touches the multipliers
+    const bool tables = mbar_wait_bounded(&tbar, 0, kWaitLimit);
     bool ok = tables;
     if (first_zero) {
         for (int i = tid; i < ntets; i += nt) slam[i] = make_float2(0.f, 0.f);
@@ -432,27 +434,24 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         asm volatile("bar.sync 1, %0;" ::"r"(MULTI ? kClusterThreads : 32 * (cw + 1)) : "memory");
     };
     const BlockVerts<MULTI> bv{sv, sw, rem, nb};
+    int staged = nne > 0 ? 1 : 0;  // copies issued (the producer's first lane counts them)
     if (MULTI || wid <= producer) {
-        int seq = 0, staged = nne > 0 ? 1 : 0;  // copies issued (the producer's first lane counts them)
+        int seq = 0;
         for (int it = 0; it < iters; it++) {
             for (int pc = 0; pc < passes * s.ncol; pc++) {
                 const int pass = SEPARATE && pc >= s.ncol ? 1 : 0, c = pc - pass * s.ncol;
                 const int4 rg = srg[c];
                 const int n = rg.y;
                 if (wid == producer) {
-                    // The next colour's records into the other buffer, whose readers passed the
-                    // last barrier. They waited for the copy before it in that buffer, unless a
-                    // wait of theirs gave up: so it is waited for here too (it has landed), and
-                    // nothing is staged after one that has not.
+                    // The next colour's records into the other buffer, whose readers passed the last
+                    // barrier, and before it waited for the copy that this one follows; after a wait
+                    // that ran out nothing is staged any more.
                     if (!s.resident && n > 0) {
-                        if (lane == 0 && seq + 1 < total && ok) {
-                            if (seq > 0) ok = mbar_wait_bounded(&bar[(seq - 1) & 1], ((seq - 1) >> 1) & 1, kWaitLimit);
-                            if (ok) {
-                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                                copy_records(sne[(seq + 1) % nne], rec + ((seq + 1) & 1) * 3 * (size_t)s.rec_cap,
-                                             &bar[(seq + 1) & 1]);
-                                staged = seq + 2;
-                            }
+                        if (lane == 0 && seq + 1 < total && !*(volatile int*)&s_stop) {
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                            copy_records(sne[(seq + 1) % nne], rec + ((seq + 1) & 1) * 3 * (size_t)s.rec_cap,
+                                         &bar[(seq + 1) & 1]);
+                            staged = seq + 2;
                         }
                         seq++;
                     }
@@ -468,8 +467,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                     const float4* buf = rec;
                     int rsub = 0;
                     if (!s.resident) {
-                        ok = __all_sync(0xffffffffu,
-                                        ok && mbar_wait_bounded(&bar[seq & 1], (seq >> 1) & 1, kWaitLimit)) != 0;
+                        // a warp that skips its work still waits for the copy: the buffer is written again
+                        const bool landed =
+                            __all_sync(0xffffffffu, mbar_wait_bounded(&bar[seq & 1], (seq >> 1) & 1, kWaitLimit)) != 0;
+                        if (!landed) s_stop = 1;
+                        ok = ok && landed;
                         buf = rec + (seq & 1) * 3 * (size_t)s.rec_cap;
                         rsub = rg.w;
                         seq++;
@@ -583,17 +585,18 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
                 }
             }
         }
-        // no block leaves with a copy into it in flight (after a wait that gave
-        // up there may be: the last one in each buffer)
-        if (wid == producer && lane == 0)
-            for (int k = staged > 1 ? staged - 2 : 0; k < staged; k++)
-                ok = mbar_wait_bounded(&bar[k & 1], (k >> 1) & 1, kWaitLimit) && ok;
     }
     // a copy or a neighbour's vertex that never came: counted; the work after it
-    // was skipped (the tables get a last bounded chance)
-    if (!__syncthreads_and(ok) && tid == 0) {
-        atomicAdd(&flags->timeouts, 1ull);
-        if (!tables) mbar_wait_bounded(&tbar, 0, kWaitLimit);
+    // was skipped, and the copies get a last bounded chance: no block leaves with
+    // one into it in flight
+    if (!__syncthreads_and(ok)) {
+        if (tid == 0) {
+            atomicAdd(&flags->timeouts, 1ull);
+            mbar_wait_bounded(&tbar, 0, kWaitLimit);
+        }
+        if (wid == producer && lane == 0)
+            for (int k = staged > 1 ? staged - 2 : 0; k < staged; k++)  // the last in each buffer
+                mbar_wait_bounded(&bar[k & 1], (k >> 1) & 1, kWaitLimit);
     }
     if (MULTI) cluster_sync_all();  // the other blocks' last stores are here
     // owners write the vertices back; every block its multipliers
