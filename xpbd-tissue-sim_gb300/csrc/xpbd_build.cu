@@ -510,6 +510,14 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
             for (int i = 0; i < 3; i++) ps.centre[3 * (size_t)q + i] += X[3 * (size_t)pv(q, k) + i] / n;
         }
     }
+    ClusterPartition part_of(ps);
+    const std::vector<int>& block = part_of.block;
+    std::vector<int> cnt, pcol;
+    // self-collisions take their own launches between the sweeps: one block only
+    const std::vector<ClusterChoice> choices =
+        part_of.choices(kClusterLanes, kMaxClusterSize, sms, c->prm.self_collisions != 0, separate ? 1.65 : 1.1,
+                        separate ? 2.2 : 1.4, separate ? 2.9 : 2.2);
+    if (choices.empty()) return XPBD_OK;
     // per patch and vertex slot the patches around the vertex and those of a
     // lower colour (slot order is colour order, and a colour holds a vertex once)
     std::vector<int> deg(V, 0);
@@ -534,19 +542,10 @@ int build_cluster(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vector
         for (int k = 0; k < kMaxPatchVerts; k++)
             for (int q = q0; q < std::min(P, q0 + 32); q++)
                 if (k < (pmeta[q].y >> 8) && rank[pv(q, k)] < 0) rank[pv(q, k)] = ranks++;
-    ClusterPartition part_of(ps);
-    const std::vector<int>& block = part_of.block;
-    std::vector<int> cnt, pcol;
-    const double other = separate ? 2.9 : 2.2;
-    // self-collisions take their own launches between the sweeps: one block only
-    const std::vector<ClusterChoice> choices =
-        part_of.choices(kClusterLanes, kMaxClusterSize, sms, c->prm.self_collisions != 0, separate ? 1.65 : 1.1,
-                        separate ? 2.2 : 1.4, other);
     int too_wide = INT_MAX;  // clusters of this many blocks did not all fit the device
     const int colours = ncol;
     const std::vector<int>& colour_of = ps.colour;
     for (const ClusterChoice& ch : choices) {
-        if (ch.us >= other * colours) break;
         if (ch.n >= too_wide) continue;
         ncol = colours;
         pcol = colour_of;

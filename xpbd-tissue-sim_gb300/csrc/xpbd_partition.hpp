@@ -80,11 +80,11 @@ public:
         return false;
     }
 
-    // The divisions that may pay and hold a vertex in two blocks at most, best first. Per round of at most `lanes`
-    // patches a block and colour a sweep takes `one` us with one block, `more`
-    // with several (and 0.75 where it waits for another block); `other` us a
-    // colour is what the route it stands in for takes. most: blocks of a cluster
-    // at most; sms: multiprocessors; single: one block only.
+    // The divisions that pay and hold a vertex in two blocks at most, best first.
+    // Per round of at most `lanes` patches a block and colour a sweep takes `one`
+    // us with one block, `more` with several (and 0.75 where it waits for another
+    // block); `other` us a colour is what the route it stands in for takes. most:
+    // blocks of a cluster at most; sms: multiprocessors; single: one block only.
     std::vector<ClusterChoice> choices(int lanes, int most, int sms, bool single, double one, double more,
                                        double other) {
         size_t largest = 0;
@@ -94,21 +94,20 @@ public:
         std::vector<ClusterChoice> out;
         int before = 0;
         for (int n : {n_min, n_min + 1, n_min + 2, n_min + 4, most}) {
-            if (n > most || (n > 1 && single) || (s.K > 1 && s.K * n > sms) || n == before)
-                continue;
+            if (n > most || (n > 1 && single) || (s.K > 1 && s.K * n > sms) || n == before) continue;
             before = n;
             for (int shape = 0; shape < 4; shape++) {
                 if ((n == 1 && shape > 0) || (shape == 3 && (n & (n - 1)))) continue;
                 assign(shape, n);
-                if (n > 2 && crowded()) continue;
                 double us = 0;
                 for (int col = 0; col < s.ncol; col++) {
                     int worst = 1;
                     for (int b = 0; b < s.K * n; b++) worst = std::max(worst, count[(size_t)b * s.ncol + col]);
                     us += (n == 1 ? one : more) * ((worst + lanes - 1) / lanes);
                 }
-                if (us < other * s.ncol && n > 1) us += 0.75 * stalls();
-                out.push_back(ClusterChoice{us, n, shape});
+                if (us >= other * s.ncol || (n > 2 && crowded())) continue;
+                if (n > 1) us += 0.75 * stalls();
+                if (us < other * s.ncol) out.push_back(ClusterChoice{us, n, shape});
             }
         }
         std::stable_sort(out.begin(), out.end(),
