@@ -90,7 +90,18 @@ static PatchSet cloud(int n) {
 
 int main(int argc, char** argv) {
     const int K = std::atoi(argv[1]), nx = std::atoi(argv[2]), ny = std::atoi(argv[3]), nz = std::atoi(argv[4]);
-    const PatchSet s = K ? grid(K, nx, ny, nz) : cloud(nx);
+    const PatchSet s = K ? grid(std::abs(K), nx, ny, nz) : cloud(nx);
+    if (K < 0) {  // whether runs of 32 patches keep the colours in step
+        std::vector<std::pair<long long, long long>> share(s.ncol, {0, 0});
+        std::vector<int> pos(s.patches());
+        for (int q = 0; q < s.patches(); q++) {
+            if (share[s.colour[q]].second++ == 0) share[s.colour[q]].first = q;
+            const double* c = &s.centre[3 * (size_t)q];
+            pos[q] = 5 * ((int)c[2] + nz * ((int)c[0] + nx * (int)c[1]));
+        }
+        std::printf("%d", (int)runs_keep_step(share, 32, 5.0 * nx * ny * nz, [&](long long q) { return pos[q]; }));
+        return 0;
+    }
     ClusterPartition p(s);
     for (int n = 1; n <= 16; n++)
         for (int shape = 0; shape < 4; shape++) {
@@ -211,3 +222,13 @@ def test_small_instances_share_tasks_only_where_that_saves_rounds(grouper, name,
         assert len(first) == len(counts) + 1
     if name in ("tiny", "just_over") and warps > 1:
         assert got < alone
+
+
+@pytest.mark.parametrize("dims,runs", [((48, 48, 48), 1), ((26, 60, 26), 1), ((36, 35, 36), 1), ((36, 27, 28), 1),
+                                       ((2, 2, 2), 1), ((35, 36, 36), 0), ((36, 36, 35), 0), ((16, 16, 15), 0),
+                                       ((47, 49, 45), 0), ((29, 29, 28), 0)])
+def test_runs_of_32_patches_only_where_they_keep_the_colours_in_step(planner, dims, runs):
+    """The mesh order runs along z, then x, then y: an odd number of hexes along y
+    ends some colours a layer earlier, along x or z it lets them drift apart."""
+    r = subprocess.run([planner, "-1", *map(str, dims)], capture_output=True, text=True)
+    assert r.returncode == 0 and int(r.stdout) == runs, r.stderr

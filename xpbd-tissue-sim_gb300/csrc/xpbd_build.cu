@@ -176,14 +176,17 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
     const int warps = per_sm * sms * ((staged ? kPatchBlock : kFlowBlock) / 32);  // co-resident
     std::vector<int4> tasks;
     std::vector<int> tcol, task_of(P);
-    // Within a group of instances, every colour in as many tasks as the largest
-    // one needs, each with an equal share of its patches (both follow the mesh
-    // order): the k-th tasks of the colours then cover the same part of the mesh,
-    // also where the colours differ in size, and a warp mostly waits for its own
-    // earlier tasks. (With runs of 32 the k-th tasks drift apart: per colour of a
-    // sweep 3.95 against 1.96 us for 16 x 16 x 15 hexes, 3.90 against 2.80 for 47
-    // x 49 x 45, the same for 48 x 48 x 48; shares of the union of 96 uneven
-    // instances instead of each one's: 4.17 against 3.99 ms a pass.) Small
+    // Within a group of instances every colour has as many tasks as the largest
+    // one needs, and the k-th tasks of the colours are to cover the same part of
+    // the mesh, so that a warp mostly waits for its own earlier tasks. Runs of 32
+    // patches do where they keep the colours in step (runs_keep_step: the same
+    // colours everywhere, or an odd number of layers along the mesh order's
+    // slowest axis); elsewhere they drift apart, and a colour goes into equal
+    // shares. 20 sweeps, shares against runs: 328 against 650 us for 16 x 16 x 15
+    // hexes, 465 against 620 for 47 x 49 x 45, but 507 against 452 for 64 x 63 x
+    // 64, 419 against 406 for 36 x 27 x 28 and 416 against 407 for 26 x 26 x 26
+    // (full runs start on whole cache lines); shares of the union of 96 uneven
+    // instances instead of each one's: 4.17 against 3.99 ms a pass. Small
     // instances share tasks where one each would take the warps more rounds
     // (task_groups): a substep of 20 sweeps of 5,000 instances of 40 hexes, five
     // lanes a task in five rounds, took 1,790 us, shares of the union 426.
@@ -208,12 +211,22 @@ int build_flow_tasks(xpbd_ctx* c, const std::vector<int4>& pmeta, const std::vec
     for (int col = 0; col < ncol; col++)
         for (int g = 0; g < G; g++)
             per_colour[g] = std::max(per_colour[g], (int)((patches(col, g).second + kTaskPatches - 1) / kTaskPatches));
+    std::vector<char> runs(G);
+    for (int g = 0; g < G; g++) {
+        std::vector<std::pair<long long, long long>> share;
+        for (int col = 0; col < ncol; col++) share.push_back(patches(col, g));
+        runs[g] = runs_keep_step(share, kTaskPatches, (double)(c->toff[group[g + 1]] - c->toff[group[g]]),
+                                 [&](long long q) { return c->tet_of_slot[pmeta[q].x]; });
+    }
     for (int col = 0; col < ncol; col++)
         for (int g = 0; g < G; g++) {
             const auto [q0, share] = patches(col, g);
+            auto cut = [&, share = share](long long i) {
+                return runs[g] ? std::min(share, kTaskPatches * i) : share * i / per_colour[g];
+            };
             for (int i = 0; i < per_colour[g]; i++) {
-                const int q = (int)(q0 + share * i / per_colour[g]);
-                const int n = (int)(q0 + share * (i + 1) / per_colour[g]) - q;
+                const int q = (int)(q0 + cut(i));
+                const int n = (int)(q0 + cut(i + 1)) - q;
                 int slots = 0;
                 for (int j = 0; j < n; j++) {
                     task_of[q + j] = (int)tasks.size();

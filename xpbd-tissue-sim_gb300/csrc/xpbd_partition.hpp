@@ -2,7 +2,9 @@
 // cluster, and which divisions are worth trying. Host C++ alone: no CUDA.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
+#include <utility>
 #include <vector>
 
 namespace xg {
@@ -222,6 +224,28 @@ inline std::vector<int> task_groups(const std::vector<std::vector<int>>& count, 
         if (cap > all) break;
     }
     return best;
+}
+
+// Whether runs of `lanes` patches keep the colours of a group in step: the k-th
+// runs of two colours lie at the same distance in the mesh for every k, to an
+// eighth of a run's extent. share: per colour its first patch and how many; pos:
+// a patch's place in the mesh order; total: the places of the group.
+template <typename Pos>
+bool runs_keep_step(const std::vector<std::pair<long long, long long>>& share, int lanes, double total, Pos pos) {
+    size_t ref = 0;
+    for (size_t c = 1; c < share.size(); c++)
+        if (share[c].second > share[ref].second) ref = c;
+    double off = 0;  // summed distances from each colour's mean one
+    for (const auto& s : share) {
+        const long long runs = (s.second + lanes - 1) / lanes;
+        auto distance = [&](long long k) {
+            return (double)(pos(s.first + lanes * k) - pos(share[ref].first + lanes * k));
+        };
+        double mean = 0;
+        for (long long k = 0; k < runs; k++) mean += distance(k) / (double)runs;
+        for (long long k = 0; k < runs; k++) off += std::abs(distance(k) - mean);
+    }
+    return off * 8 <= total * (double)share.size();  // off / (most colours) against total / most / 8
 }
 
 }  // namespace host
