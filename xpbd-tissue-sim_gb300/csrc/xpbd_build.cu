@@ -3,8 +3,8 @@
 // (ElementConstraint.hpp:23-51, HydrostaticConstraint.cpp:15-16,
 // DeviatoricConstraint.cpp:13, ElasticMaterial.hpp:31-32,
 // XPBDMeshObject.cpp:277-331), and builds the Gauss-Seidel patches and
-// colours, the dataflow tasks, the Jacobi CSR, the contact tables and the
-// self-collision grid.
+// colours, the dataflow tasks, the on-chip sweep's tables, the Jacobi blocks, the
+// contact tables and the self-collision grid.
 #include <cuda_runtime.h>
 
 #include <algorithm>

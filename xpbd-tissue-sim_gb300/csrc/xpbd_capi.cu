@@ -217,10 +217,13 @@ bool use_one_launch(const xpbd_ctx* c) {
            (p.gs_variant == 2 || p.gs_variant == 3 || p.gs_variant == 4) && c->ntasks > 0;
 }
 
-// A mesh whose largest colour is at most one warp of patches keeps the inertial
-// move, the copies into and out of the sweep's records and the velocities in
-// their own launches: the number of launches a substep of such a mesh makes is
-// part of what the interface reports (xpbd_launch_count).
+// A mesh without faces whose largest colour is at most one warp of patches keeps
+// the inertial move, the copies into and out of the versioned sweep's records and
+// the velocities in their own launches, about 1 us each of a substep. The kernel
+// does not need that: it keeps the number of launches of a substep
+// (xpbd_launch_count) what it is by the versioned sweep, from which
+// tests/test_gpu_parity.py tells on such a mesh that variant 4 does not fall back
+// to variant 2.
 bool cluster_fused(const xpbd_ctx* c) { return c->F > 0 || !c->flow_versioned || c->flow_grid > 1; }
 
 // One sweep over the tets between launches that need the positions (contacts,

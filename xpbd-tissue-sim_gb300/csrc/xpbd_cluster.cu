@@ -6,9 +6,9 @@
 // and the versioned sweep (xpbd_kernels.cu); the results agree bit for bit.
 //
 // Measured on GB300, per substep against the versioned sweep with its launches
-// around it: the 5,000-tet cube at 10 sweeps 187 -> 106 us (one block, 1.09 us a
-// colour), the 50,000-tet beam at 20 sweeps with a sphere's contacts 680 -> 413
-// us (12 blocks, 1.5 us). Tried for the exchange between blocks and slower, per
+// around it: the 5,000-tet cube at 10 sweeps 187 -> 105 us (one block, 1.09 us a
+// colour), the 50,000-tet beam at 20 sweeps with a sphere's contacts 680 -> 400
+// us (10 blocks, 1.5 us). Tried for the exchange between blocks and slower, per
 // colour of 126 patches a block: a cluster barrier with the stores in the
 // projecting lanes 2.1 us, vertices counted on an mbarrier (st.async) 2.9 us.
 #include "xpbd_device.cuh"

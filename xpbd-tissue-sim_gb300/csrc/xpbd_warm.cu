@@ -123,8 +123,8 @@ void enqueue_adam(xpbd_ctx* c, float lr) {
     c->launches += 2;
 }
 
-// Device buffers of a call on host rows. Calls of up to kKeptRows rows (44 bytes
-// each, 46 MB) share the context's, which grow to the largest such call and go
+// Device buffers of a call on host rows. Calls of up to kKeptRows rows (48 bytes
+// each, 50 MB) share the context's, which grow to the largest such call and go
 // with the context; a larger call has its own.
 constexpr int64_t kKeptRows = 1 << 20;
 struct RowBuffers {
